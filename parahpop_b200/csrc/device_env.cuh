@@ -36,13 +36,14 @@ constexpr int kMaxExpBands = 16;
 enum BodyFlag : int { kGravity = 1, kShape = 2, kRadiation = 4, kAtmosphere = 8, kOcculting = 16, kOblateness = 32 };
 
 struct DevEnv {
-    // geopotential (normalised), triangle n(n+1)/2+m, device pointers
-    int shDegree, shOrder, shNormalized;
+    // geopotential
+    int shDegree;
     double shR, shGM;
     double tideScale[7];  // converts tide-model dC/dS (SI constants) to the field's GM and radius
-    const double* shC;
-    const double* shS;
-    const double* shFac;  // interleaved (a_nm | c_m, b_nm)
+    // per tide slot: 1 for a fully normalised field, 1 / N_nm for an
+    // unnormalised one (the deltas join its coefficients as they are), 0
+    // beyond the field's degree or order
+    double tideNorm[tidefield::kSlots];
     // bodies, sorted by NAIF id (Bodies.h:105-120)
     int nbodies;
     int bodyId[kMaxBodies];

@@ -1054,20 +1054,6 @@ static T* upload(std::vector<void*>& owned, const std::vector<T>& v) {
     return d;
 }
 
-static double factorA(int n, int m, bool norm) {
-    const double nn = n, mm = m;
-    return norm ? std::sqrt(((2.0 * nn - 1.0) * (2.0 * nn + 1.0)) / ((nn - mm) * (nn + mm))) : (2.0 * nn - 1.0) / (nn - mm);
-}
-static double factorB(int n, int m, bool norm) {
-    const double nn = n, mm = m;
-    return norm ? std::sqrt(((2.0 * nn + 1.0) * (nn + mm - 1.0) * (nn - mm - 1.0)) / ((2.0 * nn - 3.0) * (nn + mm) * (nn - mm)))
-                : (nn + mm - 1.0) / (nn - mm);
-}
-static double factorC(int m, bool norm) {
-    if (norm) return m == 1 ? std::sqrt(3.0) : (m == 0 ? 1.0 : std::sqrt((2.0 * m + 1.0) / (2.0 * m)));
-    return (m == 1 || m == 0) ? 1.0 : (2.0 * m - 1.0);
-}
-
 static std::atomic<uint64_t> g_engineSerial{0};
 
 Engine::Engine(const HostEnvironment& env, int device) : host_(env), serial_(++g_engineSerial), device_(device) {
@@ -1088,7 +1074,6 @@ Engine::~Engine() {
     for (auto& kv : tiles_) {
         cudaFree(kv.second.dTile);
         cudaFree(kv.second.dBlocks);
-        cudaFree(kv.second.dDiagStep);
     }
 }
 
@@ -1097,8 +1082,6 @@ void Engine::uploadEnvironment() {
     DevEnv& e = denv_;
     std::memset(&e, 0, sizeof e);
     e.shDegree = h.hasShape ? h.shDegree : 0;
-    e.shOrder = h.hasShape ? h.shOrder : 0;
-    e.shNormalized = h.shNormalized;
     e.shR = h.shR;
     e.shGM = h.shGM;
     // tide coefficients are defined with the tide model's GM and radius: they
@@ -1110,28 +1093,15 @@ void Engine::uploadEnvironment() {
         e.tideScale[n] = h.hasShape && h.shBodyId == 399
                              ? (tidefield::kMuEarth * 1e-9 / h.shGM) * std::pow(tidefield::kRadius * 1e-3 / h.shR, (double)n)
                              : 1.0;
-    if (h.hasShape) {
-        e.shC = upload(owned_, h.shC);
-        e.shS = upload(owned_, h.shS);
-        LowTable low{};
-        for (int n = 0; n <= kLowMax + 1 && n <= h.shDegree; ++n)
-            for (int m = 0; m <= n && m <= h.shOrder; ++m) {
-                const int ti = n * (n + 1) / 2 + m;
-                if (n <= kLowMax) {
-                    low.C[ti] = h.shC[ti];
-                    low.S[ti] = h.shS[ti];
-                }
-                if (n > m) {
-                    low.a[ti] = factorA(n, m, h.shNormalized);
-                    low.b[ti] = factorB(n, m, h.shNormalized);
-                }
-            }
-        std::vector<LowTable> lv(1, low);
-        dLow_ = upload(owned_, lv);
-        std::vector<double> diag((size_t)h.shOrder + 2, 0.0);
-        for (int m = 0; m <= h.shOrder + 1; ++m) diag[m] = factorC(m, h.shNormalized);
-        dDiag_ = upload(owned_, diag);
+    const bool joined = h.hasShape && h.shBodyId == 399;
+    for (int slot = 0; slot < tidefield::kSlots; ++slot) {
+        int n, m;
+        tidefield::slotDegreeOrder(slot, n, m);
+        e.tideNorm[slot] = !joined ? 1.0
+                           : n > h.shDegree || m > h.shOrder ? 0.0
+                           : h.shNormalized ? 1.0 : 1.0 / normFactor(n, m);
     }
+    columns_ = h.hasShape ? fieldOrder(h) + 2 : 0;
     e.nbodies = (int)h.bodies.size();
     e.sunIndex = e.moonIndex = e.earthIndex = -1;
     int anyOcc = 0;
@@ -1305,72 +1275,19 @@ void Engine::uploadEnvironment() {
     e.eop = upload(owned_, h.eop);
 }
 
-// Lane-interleaved coefficient tile for the n > 8 part (layout in propagate.cuh)
+// Coefficient tile of the geopotential for L lanes (layout in geopotential.hpp)
 const Engine::Tile& Engine::tileFor(int L, bool split, int lowDeg) {
     const int key = (lowDeg * 32 + L) * 2 + (split ? 1 : 0);
     auto it = tiles_.find(key);
     if (it != tiles_.end()) return it->second;
-    const HostEnvironment& h = host_;
-    const int N = h.shDegree, M = h.shOrder;
-    const bool norm = h.shNormalized != 0;
-    const int nb = h.hasShape ? (M + 1 + L - 1) / L : 0;
-    std::vector<int2> blocks(nb > 0 ? nb : 1, int2{0, 0});
-    std::vector<TileD> entries;
-    for (int b = 0; b < nb; ++b) {
-        const int n0b = std::max(b * L, lowDeg + 1);
-        const int len = std::max(0, N - n0b + 1);
-        blocks[b] = int2{(int)entries.size(), len};
-        const size_t base = entries.size();
-        entries.resize(base + (size_t)len * L, TileD{0, 0, 0, 0, 0, 0});
-        for (int j = 0; j < L; ++j) {
-            const int m = b * L + j;
-            if (m > M) continue;
-            const int n0 = std::max(m, lowDeg + 1);
-            for (int i = 0; i < len; ++i) {
-                const int n = n0 + i;
-                if (n > N) break;
-                TileD& t = entries[base + (size_t)i * L + j];
-                const size_t ti = (size_t)n * (n + 1) / 2 + m;
-                t.c = h.shC[ti];
-                t.s = m > 0 ? h.shS[ti] : 0.0;
-                t.cp = (double)(n + 1) * t.c;
-                t.sp = (double)(n + 1) * t.s;
-                if (n + 1 <= N) {
-                    t.a = factorA(n + 1, m, norm);
-                    t.b = factorB(n + 1, m, norm);
-                }
-            }
-        }
-    }
+    const HostTile h = buildTile(host_, L, split, lowDeg);
     Tile tile;
-    tile.nblocks = nb;
-    std::vector<unsigned char> bytes;
-    if (split) {
-        std::vector<TileF> f(entries.size());
-        for (size_t k = 0; k < entries.size(); ++k)
-            f[k] = TileF{(float)entries[k].c, (float)entries[k].s, (float)entries[k].cp, (float)entries[k].sp,
-                         (float)entries[k].a, (float)entries[k].b, 0.f, 0.f};
-        bytes.resize(f.size() * sizeof(TileF));
-        std::memcpy(bytes.data(), f.data(), bytes.size());
-    } else {
-        bytes.resize(entries.size() * sizeof(TileD));
-        std::memcpy(bytes.data(), entries.data(), bytes.size());
-    }
-    bytes.resize((bytes.size() + 15) / 16 * 16 + 16, 0);
-    tile.bytes = (int)bytes.size();
-    PHOP_CUDA(cudaMalloc(&tile.dTile, bytes.size()));
-    PHOP_CUDA(cudaMemcpy(tile.dTile, bytes.data(), bytes.size(), cudaMemcpyHostToDevice));
-    PHOP_CUDA(cudaMalloc(&tile.dBlocks, blocks.size() * sizeof(int2)));
-    PHOP_CUDA(cudaMemcpy(tile.dBlocks, blocks.data(), blocks.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    // diagonal block factors D_m = c_{m+1} ... c_{m+L} and D_m (m+L)/m
-    std::vector<double2> diagStep((size_t)M + 1, double2{0.0, 0.0});
-    for (int m = 0; m + L <= M; ++m) {
-        double d = 1.0;
-        for (int k = m + 1; k <= m + L; ++k) d *= factorC(k, norm);
-        diagStep[m] = double2{d, m > 0 ? d * ((double)(m + L) / (double)m) : d};
-    }
-    PHOP_CUDA(cudaMalloc(&tile.dDiagStep, diagStep.size() * sizeof(double2)));
-    PHOP_CUDA(cudaMemcpy(tile.dDiagStep, diagStep.data(), diagStep.size() * sizeof(double2), cudaMemcpyHostToDevice));
+    tile.nblocks = h.nblocks;
+    tile.bytes = (int)h.bytes.size();
+    PHOP_CUDA(cudaMalloc(&tile.dTile, h.bytes.size()));
+    PHOP_CUDA(cudaMemcpy(tile.dTile, h.bytes.data(), h.bytes.size(), cudaMemcpyHostToDevice));
+    PHOP_CUDA(cudaMalloc(&tile.dBlocks, h.blocks.size() * sizeof(int4)));
+    PHOP_CUDA(cudaMemcpy(tile.dBlocks, h.blocks.data(), h.blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return tiles_.emplace(key, tile).first->second;
 }
 
@@ -1560,8 +1477,8 @@ void Engine::launchStepGraph(const StepParams& p, const LaunchShape& shape, cons
     PHOP_CUDA(cudaGraphLaunch(key.exec, stream));
 }
 
-// FP64 low part of each column: n <= 8 in the FP64 form, n <= the option's
-// degree in split precision.  Its default follows the field's degree: the
+// FP64 low part of each column in split precision (the FP64 form ignores
+// it): n <= the option's degree.  Its default follows the field's degree: the
 // FP32 rounding of the recursion accumulates over more terms in a larger
 // field (24 h, 10^5 LEO objects at degree 120: 11.5 mm max with n <= 20 in
 // FP64, 8.3 mm with n <= 24; degree 70: 6.4 mm with n <= 20).
@@ -1586,12 +1503,17 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     p.tileBytes = tile.bytes;
     p.blocks = tile.dBlocks;
     p.nblocks = tile.nblocks;
-    p.diagStep = tile.dDiagStep;
+    p.columns = columns_;
     p.lowDeg = lowDeg;
     p.tile64 = nullptr;
+    p.blocks64 = nullptr;
+    p.nblocks64 = 0;
     p.splitRadius = 0.0;
     if (opt.split && opt.splitFloorKm > 0.0) {
-        p.tile64 = tileFor(L, false, lowDeg).dTile;
+        const Tile& full = tileFor(L, false, lowDeg);
+        p.tile64 = full.dTile;
+        p.blocks64 = full.dBlocks;
+        p.nblocks64 = full.nblocks;
         p.splitRadius = host_.shR + opt.splitFloorKm;
     }
     // shared memory per CTA: the coefficient tile (when it fits) plus the
@@ -1760,8 +1682,6 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
     p.state = dState;
     p.bc = dBc;
     p.ams = dAms;
-    p.low = dLow_;
-    p.diagC = dDiag_;
     p.maxSteps = maxSteps;
     p.order = dOrder;
     p.cur = g.cur;

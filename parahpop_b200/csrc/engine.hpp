@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "device_env.cuh"
+#include "geopotential.hpp"
 #include "propagate.cuh"
 #include "value.hpp"
 
@@ -155,7 +156,7 @@ struct RunOptions {
     int trajRecords = 0;  // capacity of dTraj in records
 };
 
-// degrees n <= this of every column run in FP64 from the LowTable
+// split precision: degrees n <= this run in FP64
 int lowDegreeFor(const RunOptions& opt, int fieldDegree);
 
 class Engine {
@@ -201,15 +202,9 @@ public:
                           double* outEpochMjd, cudaStream_t stream = 0);
 
     // internal
-    struct HostTile {
-        std::vector<unsigned char> bytes;
-        std::vector<int2> blocks;
-        int nblocks = 0;
-    };
     struct Tile {
         void* dTile = nullptr;
-        int2* dBlocks = nullptr;
-        double2* dDiagStep = nullptr;
+        int4* dBlocks = nullptr;
         int bytes = 0;
         int nblocks = 0;
     };
@@ -280,8 +275,7 @@ private:
     std::map<std::string, std::pair<void*, size_t>> scratch_;
     std::map<int, Tile> tiles_;
     std::map<int, HostTile> hostTiles_;
-    LowTable* dLow_ = nullptr;
-    double* dDiag_ = nullptr;
+    int columns_ = 0;  // orders 0 .. columns_ - 1 of the geopotential tile have rows
     std::map<int, int> tuned_;  // autotuned lane count per batch class
     std::map<int64_t, int> occupancy_;  // resident CTAs per SM by launch configuration
     std::map<int, std::pair<int, int>> attrs_;  // maxThreadsPerBlock, numRegs of each step-kernel instantiation

@@ -1,0 +1,72 @@
+// Coefficient tile of the geopotential and its host-side construction.
+//
+// The acceleration of a spherical-harmonic field is itself a sum of solid
+// harmonics, one degree and one order further: with the column functions
+// p_nu,M = alpha^nu P_nu,M(sin phi) (alpha = R / r, fully normalised),
+//     a_x = GM / R^2 alpha sum_M cos M lambda sum_nu Xc p + sin M lambda sum_nu Xs p
+// and likewise a_y (Yc, Ys) and a_z (Zc, Zs), where row nu of column M holds
+// constants formed here from C, S of degree n = nu - 1 and orders M - 1, M,
+// M + 1 (Montenbruck & Gill, Satellite Orbits, 2000, section 3.2.5; the
+// reference sums the same field term by term in spherical components,
+// DegreeLoop.h:83-112).  One term is then one step of one recurrence and six
+// sums, without latitude derivatives and without a division by cos phi.
+//
+// The recurrence p_{nu+1} = a alpha s p_nu - b alpha^2 p_{nu-1} is scaled
+// per column (p = sigma q, sigma_{nu+1} = b sigma_{nu-1}) to
+//     q_{nu+1} = A alpha s q_nu - alpha^2 q_{nu-1},
+// so a row carries one recurrence factor A and six coefficients (x sigma).
+// sigma_M = P_MM / cos^M phi, so a column starts from q_M = (alpha cos phi)^M.
+//
+// Layout: columns 0 .. order + 1 in blocks of W (W lanes, lane j takes column
+// b W + j), rows in pairs.  A row pair of a lane is seven 16-byte chunks in
+// FP64 (A0 A1 | Xc0 Xs0 | Yc0 Ys0 | Zc0 Zs0 | Xc1 Xs1 | Yc1 Ys1 | Zc1 Zs1)
+// and four in FP32 (A0 A1 Xc0 Xs0 | Yc0 Ys0 Zc0 Zs0 | Xc1 Xs1 Yc1 Ys1 |
+// Zc1 Zs1 - -), chunk c of pair i of lane j at ((i chunks + c) W + j): the
+// lanes of a load read consecutive 16-byte words.  In split precision the
+// rows of degrees n <= lowDeg come first, as FP64 pairs (rounded up to whole
+// pairs), the others as FP32 pairs.
+#pragma once
+#include <vector_types.h>
+
+#include <vector>
+
+#if defined(__CUDACC__)
+#define PHOP_GEO_HD __host__ __device__ __forceinline__
+#else
+#define PHOP_GEO_HD inline
+#endif
+
+namespace phop {
+
+constexpr int kChunks64 = 7;  // 16-byte chunks of an FP64 row pair
+constexpr int kChunks32 = 4;  // and of an FP32 row pair
+
+// FP64 and FP32 row pairs of column M in a field of degree N whose FP64 low
+// part is `lowDeg` (lowDeg >= N: all rows)
+PHOP_GEO_HD int rowPairs64(int M, int N, int lowDeg) {
+    const int top = lowDeg + 1 < N ? lowDeg + 2 : N + 1;
+    const int rows = top - M + 1;
+    return rows > 0 ? (rows + 1) / 2 : 0;
+}
+PHOP_GEO_HD int rowPairs32(int M, int N, int lowDeg) {
+    const int rows = N + 2 - M - 2 * rowPairs64(M, N, lowDeg);
+    return rows > 0 ? (rows + 1) / 2 : 0;
+}
+
+struct HostTile {
+    std::vector<unsigned char> bytes;
+    std::vector<int4> blocks;  // per block: {first FP64 chunk, -, first FP32 chunk, -} in 16-byte units
+    int nblocks = 0;
+};
+
+struct HostEnvironment;
+
+// Tile for W lanes; split: rows above degree lowDeg in FP32.  The columns end
+// at the last order that has a nonzero coefficient (plus one).
+HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg);
+// Last order with a nonzero coefficient.
+int fieldOrder(const HostEnvironment& h);
+// N_nm of the full normalisation (C = N_nm C_normalised).
+double normFactor(int n, int m);
+
+}  // namespace phop

@@ -16,8 +16,8 @@
 //   epoch records                                13 x kMaxSteps records
 //
 // Limits: at most kMaxSteps (256) fixed steps per call and a coefficient tile
-// of at most kTileBytes (512 KiB, enough for degree/order 120 in FP64); calls
-// beyond them are rejected with an error.  Every GPU that loads the library
+// of at most 512 KiB at one entry per term (withinTileLimit; enough for
+// degree/order 120 in FP64); calls beyond them are rejected with an error.  Every GPU that loads the library
 // holds the array (4 MiB) until the process exits.  All calls share it: the
 // control words are cleared on every call, the tile is re-copied whenever a
 // call needs another one than the array holds (keyed by the context's
@@ -43,7 +43,7 @@ namespace phop {
 constexpr size_t kStaticScratchBytes = 4u << 20;
 constexpr int kMaxSteps = 256;
 constexpr size_t kCtlBytes = 256;
-constexpr size_t kTileBytes = 512u << 10;
+constexpr size_t kTileBytes = 640u << 10;
 constexpr size_t kBlockBytes = 4u << 10;
 
 static __device__ __align__(256) unsigned char g_staticScratch[kStaticScratchBytes];
@@ -63,70 +63,26 @@ static_assert(kCtlBytes + kTileBytes + kBlockBytes + 2 * kMaxSteps * sizeof(doub
               "static scratch layout does not fit");
 }  // namespace
 
-// Host copy of the lane-interleaved coefficient tile (same layout as the
-// engine's device tiles, propagate.cuh), kept so the allocation-free entry
-// point can copy it into the static array without allocating.
-static double tileFactorA(int n, int m, bool norm) {
-    const double nn = n, mm = m;
-    return norm ? std::sqrt(((2.0 * nn - 1.0) * (2.0 * nn + 1.0)) / ((nn - mm) * (nn + mm))) : (2.0 * nn - 1.0) / (nn - mm);
-}
-static double tileFactorB(int n, int m, bool norm) {
-    const double nn = n, mm = m;
-    return norm ? std::sqrt(((2.0 * nn + 1.0) * (nn + mm - 1.0) * (nn - mm - 1.0)) / ((2.0 * nn - 3.0) * (nn + mm) * (nn - mm)))
-                : (nn + mm - 1.0) / (nn - mm);
-}
-
-const Engine::HostTile& Engine::hostTileFor(int L, bool split, int lowDeg) {
+// Host copy of the coefficient tile, kept so the allocation-free entry point
+// can copy it into the static array without allocating.
+const HostTile& Engine::hostTileFor(int L, bool split, int lowDeg) {
     const int key = (lowDeg * 32 + L) * 2 + (split ? 1 : 0);
     auto it = hostTiles_.find(key);
     if (it != hostTiles_.end()) return it->second;
-    const HostEnvironment& h = host_;
-    const int N = h.shDegree, M = h.shOrder;
-    const bool norm = h.shNormalized != 0;
-    const int nb = h.hasShape ? (M + 1 + L - 1) / L : 0;
-    HostTile out;
-    out.nblocks = nb;
-    out.blocks.assign(nb > 0 ? nb : 1, int2{0, 0});
-    std::vector<TileD> entries;
-    for (int b = 0; b < nb; ++b) {
-        const int n0b = std::max(b * L, lowDeg + 1);
-        const int len = std::max(0, N - n0b + 1);
-        out.blocks[b] = int2{(int)entries.size(), len};
-        const size_t base = entries.size();
-        entries.resize(base + (size_t)len * L, TileD{0, 0, 0, 0, 0, 0});
-        for (int j = 0; j < L; ++j) {
-            const int m = b * L + j;
-            if (m > M) continue;
-            const int n0 = std::max(m, lowDeg + 1);
-            for (int i = 0; i < len; ++i) {
-                const int n = n0 + i;
-                if (n > N) break;
-                TileD& t = entries[base + (size_t)i * L + j];
-                const size_t ti = (size_t)n * (n + 1) / 2 + m;
-                t.c = h.shC[ti];
-                t.s = m > 0 ? h.shS[ti] : 0.0;
-                t.cp = (double)(n + 1) * t.c;
-                t.sp = (double)(n + 1) * t.s;
-                if (n + 1 <= N) {
-                    t.a = tileFactorA(n + 1, m, norm);
-                    t.b = tileFactorB(n + 1, m, norm);
-                }
-            }
-        }
-    }
-    if (split) {
-        std::vector<TileF> f(entries.size());
-        for (size_t k = 0; k < entries.size(); ++k)
-            f[k] = TileF{(float)entries[k].c, (float)entries[k].s, (float)entries[k].cp, (float)entries[k].sp,
-                         (float)entries[k].a, (float)entries[k].b, 0.f, 0.f};
-        out.bytes.resize(f.size() * sizeof(TileF));
-        std::memcpy(out.bytes.data(), f.data(), out.bytes.size());
-    } else {
-        out.bytes.resize(entries.size() * sizeof(TileD));
-        std::memcpy(out.bytes.data(), entries.data(), out.bytes.size());
-    }
-    out.bytes.resize((out.bytes.size() + 15) / 16 * 16 + 16, 0);
-    return hostTiles_.emplace(key, std::move(out)).first->second;
+    return hostTiles_.emplace(key, buildTile(host_, L, split, lowDeg)).first->second;
+}
+
+// The entry point's size limit, stated for a tile of one 48-byte (FP64) or
+// 32-byte (split precision) entry per term above degree `lowDeg`, columns in
+// blocks of L padded to the block's longest, and 8 bytes per block.  The
+// tile in use holds more bytes per term; kTileBytes is what the largest
+// field within the limit needs (629,904 bytes, degree 145 at four lanes).
+static bool withinTileLimit(int N, int M, int L, bool split, int lowDeg) {
+    const int nb = (M + L) / L;
+    int64_t entries = 0;
+    for (int b = 0; b < nb; ++b) entries += (int64_t)std::max(0, N - std::max(b * L, lowDeg + 1) + 1) * L;
+    const int64_t bytes = (entries * (split ? 32 : 48) + 15) / 16 * 16 + 16;
+    return bytes <= (512 << 10) && nb * 8 <= (4 << 10);
 }
 
 // Device address of the static scratch array on `device` (set up once per
@@ -188,7 +144,7 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     p += kCtlBytes;
     void* tileDst = p;
     p += kTileBytes;
-    int2* blocksDst = (int2*)p;
+    int4* blocksDst = (int4*)p;
     p += kBlockBytes;
     double* dT0 = (double*)p;
     p += kMaxSteps * sizeof(double);
@@ -200,8 +156,10 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     // coefficient tile (host copy kept by the engine) into the array
     const int L = opt.lanes > 0 ? opt.lanes : autoLanes(n);
     const int lowDeg = lowDegreeFor(opt, host_.shDegree);
+    if (host_.hasShape && !withinTileLimit(host_.shDegree, host_.shOrder, L, opt.split, lowDeg))
+        throw std::runtime_error("coefficient tile exceeds the allocation-free entry point's 512 KiB limit");
     const HostTile& ht = hostTileFor(L, opt.split, lowDeg);
-    if (ht.bytes.size() > kTileBytes || ht.blocks.size() * sizeof(int2) > kBlockBytes)
+    if (ht.bytes.size() > kTileBytes || ht.blocks.size() * sizeof(int4) > kBlockBytes)
         throw std::runtime_error("coefficient tile exceeds the allocation-free entry point's 512 KiB limit");
     const int key = (lowDeg * 32 + L) * 2 + (opt.split ? 1 : 0);
     auto check = [](cudaError_t e) {
@@ -215,7 +173,7 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
         if (ds.tileOwner != serial_ || ds.tileKey != key) {
             ds.tileOwner = 0;
             check(cudaMemcpyAsync(tileDst, ht.bytes.data(), ht.bytes.size(), cudaMemcpyHostToDevice, stream));
-            check(cudaMemcpyAsync(blocksDst, ht.blocks.data(), ht.blocks.size() * sizeof(int2),
+            check(cudaMemcpyAsync(blocksDst, ht.blocks.data(), ht.blocks.size() * sizeof(int4),
                                   cudaMemcpyHostToDevice, stream));
             ds.tileOwner = serial_;
             ds.tileKey = key;
@@ -242,9 +200,8 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.tileBytes = (int)ht.bytes.size();
     sp.blocks = blocksDst;
     sp.nblocks = ht.nblocks;
-    sp.low = dLow_;
+    sp.columns = columns_;
     sp.lowDeg = lowDeg;
-    sp.diagC = dDiag_;
     sp.workCounter = ctl;
     sp.errorFlag = ctl + 1;
     const int threadsReq = std::min(opt.threads > 0 ? opt.threads : 512, maxStepThreads(L));

@@ -55,8 +55,8 @@ __global__ void __launch_bounds__(64) epochRecordsKernel(const __grid_constant__
         tidefield::tideDeltasWarp(ep, env.solid != 0, env.ocean != 0, env.zeroTide != 0, env.tideOcean,
                                   env.tideScale, dC, dS);
         if (lane < tidefield::kSlots) {
-            out[warpFirst + src].dC[lane + 3] = dC;
-            out[warpFirst + src].dS[lane + 3] = dS;
+            out[warpFirst + src].dC[lane + 3] = dC * env.tideNorm[lane];
+            out[warpFirst + src].dS[lane + 3] = dS * env.tideNorm[lane];
         }
     }
 }

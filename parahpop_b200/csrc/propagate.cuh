@@ -13,21 +13,14 @@
 //     stage state for its components in the reference's order
 //     (parm/integrate/rk/host/Step.h:33-84) and the 8th-order update in stage
 //     order (Step.h:86-104), and broadcasts components by warp shuffle.
-//   * Spherical harmonics: orders m are processed in blocks of L columns, lane
-//     j taking m = bL + j.  Every lane advances the diagonal P_mm, dP_mm,
-//     cos/sin(m lambda) and alpha^m with the reference's recurrences
-//     (LegendreRecursor.h:202-208, PseudoPhasor.h:58-64), so the column start
-//     values are the reference's.  The n <= 8 part of each column (with the
-//     epoch's tide deltas folded into n <= 6) is always FP64; the n > 8 part
-//     runs in the tile type T (double, or float for split precision) from a
-//     lane-interleaved coefficient tile that a TMA bulk copy stages into
-//     shared memory, so the L lanes of a group read one contiguous line per
-//     term and the groups of a warp share it by broadcast.  Per column the
-//     sums  sum (n+1) c Pt, sum (n+1) s Pt, sum c dPt, sum s dPt, sum c Pt,
-//     sum s Pt  (Pt = alpha^n P) are accumulated and the phasor applied once,
-//     which is algebraically the reference's per-term phase product
-//     (DegreeLoop.h:83-112).  Partial accelerations are folded across the
-//     group by xor shuffles.
+//   * Spherical harmonics: the field's acceleration as column sums of solid
+//     harmonics one degree up (geopotential.hpp), orders M in blocks of L
+//     columns (2L where two lane groups share their columns: every lane then
+//     runs its column for both groups' objects), from a lane-interleaved
+//     coefficient tile that a TMA bulk copy stages into shared memory.  In
+//     split precision the degrees above the FP64 low part run in FP32.  The
+//     Earth's tide deltas (n <= 6) are summed apart, in FP64.  Partial
+//     accelerations are folded across the group by xor shuffles.
 //   * Everything else (third bodies, SRP with shadow, NRLMSISE-00 drag,
 //     relativity) is evaluated by every lane of the group on the broadcast
 //     stage state.
@@ -46,36 +39,13 @@
 
 namespace phop {
 
-// Each column's low degrees run in FP64 from the LowTable (with the epoch's
-// tide deltas for n <= 6); the tile holds the degrees above.  The FP64 form
-// starts its tile at n = 9; split precision keeps n <= splitFp64Degree
-// (by default 20, or 24 for fields above degree 80; at most kLowMax) in FP64
-// and runs the rest in FP32.
-constexpr int kLowDeg = 8;                                  // FP64 form: n <= 8 from the LowTable
+// Split precision keeps degrees n <= splitFp64Degree (by default 20, or 24
+// for fields above degree 80; at most kLowMax) of every column in FP64 and
+// runs the rest in FP32.
+constexpr int kLowDeg = 8;                                  // smallest FP64 low part of the split form
 constexpr int kSplitFp64Degree = 20;                        // split form default up to degree 80
 constexpr int kSplitFp64DegreeHigh = 24;                    // split form default above degree 80
 constexpr int kLowMax = 24;                                 // largest FP64 low part
-constexpr int kLowTri = (kLowMax + 2) * (kLowMax + 3) / 2;  // factor triangle up to n = kLowMax + 1
-
-// coefficient tile entry for the n > 8 part: c, s, (n+1)c, (n+1)s and the
-// recursion factors a, b of the step n -> n+1
-struct __align__(16) TileD {
-    double c, s, cp, sp, a, b;
-};
-struct __align__(16) TileF {
-    float c, s, cp, sp, a, b, pad0, pad1;
-};
-template <typename T> struct TileOf;
-template <> struct TileOf<double> { using type = TileD; };
-template <> struct TileOf<float> { using type = TileF; };
-
-// low-degree FP64 table (n <= kLowMax coefficients, factors to n = kLowMax + 1)
-struct LowTable {
-    double C[kLowTri];
-    double S[kLowTri];
-    double a[kLowTri];
-    double b[kLowTri];
-};
 
 struct StepParams {
     DevEnv env;
@@ -117,13 +87,13 @@ struct StepParams {
     // geopotential
     const void* tile;       // tile entries in global memory
     int tileBytes;          // multiple of 16
-    const int2* blocks;     // per block: entry offset, length
+    const int4* blocks;     // per block of columns: first FP64 and FP32 chunk (geopotential.hpp)
     int nblocks;
-    const LowTable* low;
-    const double* diagC;    // c_m, m = 0..M
-    const double2* diagStep;  // per m: (c_{m+1}...c_{m+L}, same x (m+L)/m), nullable
-    int lowDeg;             // n <= lowDeg of every column in FP64 from `low`; the tile starts at lowDeg + 1
-    const void* tile64;     // split precision: the FP64 tile (global memory, same blocks)
+    int columns;            // orders 0 .. columns - 1 have rows
+    int lowDeg;             // split precision: rows of degrees n <= lowDeg are FP64
+    const void* tile64;     // split precision: the FP64 tile (global memory) of L lanes, its blocks
+    const int4* blocks64;
+    int nblocks64;
     double splitRadius;     // split precision: radius (km) below which the tile part stays FP64; 0 = none
     int useSmemTile;
     int pairSh;             // the geopotential of lane-group pairs (tile built for 2L lanes)

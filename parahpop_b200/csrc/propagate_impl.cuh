@@ -6,6 +6,7 @@
 
 #include <type_traits>
 
+#include "geopotential.cuh"
 #include "nrlmsise00.cuh"
 #include "propagate.cuh"
 
@@ -115,11 +116,6 @@ static __device__ __forceinline__ void finalUpdate(double (&y)[CPL], const Stage
 // local memory.
 struct RecordRef {
     const EpochRecord* r;
-    // the record of the object held by lane (lane ^ delta)
-    __device__ __forceinline__ RecordRef partner(unsigned mask, int delta) const {
-        const unsigned long long q = __shfl_xor_sync(mask, (unsigned long long)r, delta);
-        return RecordRef{(const EpochRecord*)q};
-    }
     __device__ __forceinline__ double R(int i) const { return r->R[i]; }
     __device__ __forceinline__ double W(int i) const { return r->w[i]; }
     __device__ __forceinline__ double body(int b, int i) const { return r->body[b][i]; }
@@ -145,18 +141,7 @@ struct RecordInterp {
     const double2* g;
     double w0, w1, w2, w3;
     double et;        // the stage epoch (TDB s past J2000)
-    __device__ __forceinline__ RecordInterp partner(unsigned mask, int delta) const {
-        RecordInterp o;
-        o.g = (const double2*)__shfl_xor_sync(mask, (unsigned long long)g, delta);
-        o.w0 = __shfl_xor_sync(mask, w0, delta);
-        o.w1 = __shfl_xor_sync(mask, w1, delta);
-        o.w2 = __shfl_xor_sync(mask, w2, delta);
-        o.w3 = __shfl_xor_sync(mask, w3, delta);
-        o.et = __shfl_xor_sync(mask, et, delta);
-        return o;
-    }
-    // explicit roundings: every copy of this code gives the same bits (the
-    // geopotential of lane-group pairs evaluates it for both objects)
+    // explicit roundings: every copy of this code gives the same bits
     __device__ __forceinline__ double at(int off) const {
         const double2 x = g[off], y = g[2 * kInterpFields + off];
         return __fma_rn(w3, y.y, __fma_rn(w2, y.x, __fma_rn(w1, x.y, __dmul_rn(w0, x.x))));
@@ -198,513 +183,6 @@ static __device__ __forceinline__ void fromBody(const Rec& r, const double a[3],
     out[0] = r.R(0) * a[0] + r.R(3) * a[1] + r.R(6) * a[2];
     out[1] = r.R(1) * a[0] + r.R(4) * a[1] + r.R(7) * a[2];
     out[2] = r.R(2) * a[0] + r.R(5) * a[1] + r.R(8) * a[2];
-}
-
-// ---- spherical harmonics, lane-split over orders --------------------------------------------
-template <int L, typename T, class Rec>
-static __device__ __forceinline__ void shAccel(const StepParams& p, const typename TileOf<T>::type* __restrict__ tile,
-                                        const Rec& rec, double x, double y, double z, double out[3]) {
-    using Tile = typename TileOf<T>::type;
-    const int j = (int)(threadIdx.x % L);
-    const int N = p.env.shDegree, M = p.env.shOrder;
-    const int lowDeg = p.lowDeg;
-    const bool tides = p.env.shTides != 0;
-    const LowTable* __restrict__ low = p.low;
-    const double* __restrict__ diagC = p.diagC;
-    const double rn = sqrt(x * x + y * y + z * z);
-    const double rho = sqrt(x * x + y * y);
-    const double sinPhi = z / rn, cosPhi = rho / rn;
-    const double sinL = rho > 1e-14 ? y / rho : 0.0;
-    const double cosL = rho > 1e-14 ? x / rho : 1.0;
-    const double alpha = p.env.shR / rn;
-    const double invCos = cosPhi == 0.0 ? 0.0 : 1.0 / cosPhi;
-    // diagonal state (reference recurrences) for this lane's first column
-    double Pmm = 1.0, dPmm = 0.0, cML = 1.0, sML = 0.0, am = 1.0;
-    int m = 0;
-    auto advance = [&]() {
-        const double ns = cosL * sML + sinL * cML;
-        const double nc = cosL * cML - sinL * sML;
-        sML = ns;
-        cML = nc;
-        const double cm = diagC[m + 1];
-        const double nP = cm * cosPhi * Pmm;
-        const double ndP = cm * (cosPhi * dPmm - sinPhi * Pmm);
-        Pmm = nP;
-        dPmm = ndP;
-        am *= alpha;
-        ++m;
-    };
-    for (int t = 0; t < j; ++t)
-        if (m < M) advance();
-    // block advance m -> m + L in one step where the per-L factor table is
-    // present: P_{m+L} = D_m cos^L P_m and dP_{m+L} = D'_m cos^L dP_m with
-    // D_m = c_{m+1} ... c_{m+L}, D'_m = D_m (m+L)/m (closed forms of the
-    // diagonal recurrences; m = 0 starts from dP_L = -L sin cos^{L-1} D_0), the
-    // phasor rotated by L lambda and alpha^m scaled by alpha^L.
-    const double2* __restrict__ diagStep = p.diagStep;
-    double cosL1 = 1.0, cLam = 1.0, sLam = 0.0, aL = 1.0;
-    if (L > 1 && diagStep) {
-#pragma unroll
-        for (int t = 0; t < L - 1; ++t) cosL1 *= cosPhi;
-#pragma unroll
-        for (int t = 0; t < L; ++t) {
-            const double ns = cosL * sLam + sinL * cLam;
-            const double nc = cosL * cLam - sinL * sLam;
-            sLam = ns;
-            cLam = nc;
-            aL *= alpha;
-        }
-    }
-    const double cosLp = cosL1 * cosPhi;
-    const T u = T(alpha * sinPhi), v = T(alpha * cosPhi), a2 = T(alpha * alpha);
-    double ar = 0.0, aphi = 0.0, alam = 0.0;
-    const int nblocks = p.nblocks;
-    for (int b = 0; b < nblocks; ++b) {
-        const int mcol = b * L + j;
-        const bool act = mcol <= M;
-        double SA0 = 0, SA1 = 0, SA2 = 0, SA3 = 0, SA4 = 0, SA5 = 0;
-        T P = T(0), P1 = T(0), dP = T(0), dP1 = T(0);
-        if (act && mcol <= lowDeg) {
-            // n = mcol .. lowDeg in FP64 with the epoch's tide deltas (n <= 6)
-            double Pn = Pmm, Pn1 = 0.0, dPn = dPmm, dPn1 = 0.0, an = am, anPrev = am;
-            const int nEnd = N < lowDeg ? N : lowDeg;
-            for (int n = mcol; n <= nEnd; ++n) {
-                const int ti = n * (n + 1) / 2 + mcol;
-                // order 0 has no sine term: nothing to read for it
-                double c = low->C[ti], s = mcol == 0 ? 0.0 : low->S[ti];
-                if (n <= 6 && tides) {
-                    c += rec.dC(ti);
-                    if (mcol != 0) s += rec.dS(ti);
-                }
-                const double q = an * Pn, qd = an * dPn, np1 = (double)(n + 1);
-                SA0 = fma(np1 * c, q, SA0);
-                SA1 = fma(np1 * s, q, SA1);
-                SA2 = fma(c, qd, SA2);
-                SA3 = fma(s, qd, SA3);
-                SA4 = fma(c, q, SA4);
-                SA5 = fma(s, q, SA5);
-                if (n < N) {
-                    const int tn = (n + 1) * (n + 2) / 2 + mcol;
-                    const double fa = low->a[tn], fb = low->b[tn];
-                    const double P2 = Pn1;
-                    Pn1 = Pn;
-                    Pn = fa * sinPhi * Pn1 - fb * P2;
-                    const double dP2 = dPn1;
-                    dPn1 = dPn;
-                    dPn = fa * (sinPhi * dPn1 + cosPhi * Pn1) - fb * dP2;
-                    anPrev = an;
-                    an *= alpha;
-                }
-            }
-            P = T(an * Pn);
-            P1 = T(anPrev * Pn1);
-            dP = T(an * dPn);
-            dP1 = T(anPrev * dPn1);
-        } else if (act) {
-            P = T(am * Pmm);
-            dP = T(am * dPmm);
-        }
-        // n > 8 part from the lane-interleaved tile
-        const int2 blk = p.blocks[b];
-        T Scc = T(0), Ssc = T(0), Sdc = T(0), Sds = T(0), Spc = T(0), Sps = T(0);
-        const Tile* tp = tile + blk.x + j;
-        for (int i = 0; i < blk.y; ++i, tp += L) {
-            const Tile e = *tp;
-            Scc = fma(T(e.cp), P, Scc);
-            Ssc = fma(T(e.sp), P, Ssc);
-            Spc = fma(T(e.c), P, Spc);
-            Sps = fma(T(e.s), P, Sps);
-            Sdc = fma(T(e.c), dP, Sdc);
-            Sds = fma(T(e.s), dP, Sds);
-            const T Pn = fma(T(e.a), u * P, -T(e.b) * (a2 * P1));
-            const T dPn = fma(T(e.a), fma(u, dP, v * P), -T(e.b) * (a2 * dP1));
-            P1 = P;
-            P = Pn;
-            dP1 = dP;
-            dP = dPn;
-        }
-        if (act) {
-            const double cc = SA0 + (double)Scc, sc = SA1 + (double)Ssc;
-            const double dc = SA2 + (double)Sdc, ds = SA3 + (double)Sds;
-            const double pc = SA4 + (double)Spc, ps = SA5 + (double)Sps;
-            ar -= cML * cc + sML * sc;
-            aphi += cML * dc + sML * ds;
-            alam -= ((double)mcol * invCos) * (sML * pc - cML * ps);
-        }
-        if (L > 1 && diagStep) {
-            if (m + L <= M) {
-                const double2 f = diagStep[m];
-                const double nP = f.x * cosLp * Pmm;
-                const double ndP = m == 0 ? -(double)L * sinPhi * cosL1 * f.x : f.y * cosLp * dPmm;
-                Pmm = nP;
-                dPmm = ndP;
-                const double ns = cLam * sML + sLam * cML;
-                const double nc = cLam * cML - sLam * sML;
-                sML = ns;
-                cML = nc;
-                am *= aL;
-                m += L;
-            } else {
-                m = M + 1;  // beyond the last order: the lane's later columns are inactive
-            }
-        } else {
-            for (int t = 0; t < L; ++t)
-                if (m < M) advance();
-        }
-    }
-    // fold the group's partial sums (the group's lanes only: in split
-    // precision groups of one warp may take different precisions)
-    const unsigned groupMask = L >= 32 ? 0xffffffffu : (((1u << L) - 1u) << ((threadIdx.x & 31) - j));
-#pragma unroll
-    for (int off = L / 2; off > 0; off >>= 1) {
-        ar += __shfl_xor_sync(groupMask, ar, off);
-        aphi += __shfl_xor_sync(groupMask, aphi, off);
-        alam += __shfl_xor_sync(groupMask, alam, off);
-    }
-    if (cosPhi == 0.0 && M >= 1) {
-        // exact pole: the m = 1 longitudinal term takes its analytical limit
-        // (DegreeLoop.h:98-103, Coefficients.h:123-131)
-        double an = alpha;
-        for (int n = 1; n <= N; ++n) {
-            const int ti = n * (n + 1) / 2 + 1;
-            double s = p.env.shS[ti];
-            if (n <= 6 && tides) s += rec.dS(ti);
-            const double sign = sinPhi > 0.0 ? 1.0 : ((n & 1) ? 1.0 : -1.0);
-            double lim = 0.5 * (double)n * (n + 1.0);
-            if (p.env.shNormalized) lim *= sqrt(2.0 * (2.0 * n + 1.0) / ((double)n * (n + 1.0)));
-            // S~ = c sin(l) - s cos(l) with sin(l) = 0, cos(l) = 1 at the pole
-            alam -= an * (sign * lim) * (-s);
-            an *= alpha;
-        }
-    }
-    const double g = p.env.shGM / (rn * rn);
-    ar *= g;
-    aphi *= g;
-    alam *= g;
-    out[0] = cosPhi * cosL * ar - sinPhi * cosL * aphi - sinL * alam;
-    out[1] = cosPhi * sinL * ar - sinPhi * sinL * aphi + cosL * alam;
-    out[2] = sinPhi * ar + cosPhi * aphi;
-}
-
-// ---- spherical harmonics for a pair of objects, packed FP32 ---------------------------------
-// Two FP32 values in one 64-bit register pair, operated on by the packed
-// f32x2 instructions of sm_100.
-struct F2 {
-    unsigned long long v;
-};
-static __device__ __forceinline__ F2 f2(float lo, float hi) {
-    F2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
-    return r;
-}
-static __device__ __forceinline__ F2 f2fma(F2 a, F2 b, F2 c) {
-    F2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d.v) : "l"(a.v), "l"(b.v), "l"(c.v));
-    return d;
-}
-static __device__ __forceinline__ F2 f2mul(F2 a, F2 b) {
-    F2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d.v) : "l"(a.v), "l"(b.v));
-    return d;
-}
-static __device__ __forceinline__ void f2split(F2 a, float& lo, float& hi) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
-}
-// The FP64 form of the same pair: two doubles, operated on one by one.
-struct D2 {
-    double lo, hi;
-};
-template <typename T> struct PairOf;
-template <> struct PairOf<float> {
-    using type = F2;
-    static __device__ __forceinline__ F2 make(float a, float b) { return f2(a, b); }
-    static __device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { return f2fma(a, b, c); }
-    static __device__ __forceinline__ F2 mul(F2 a, F2 b) { return f2mul(a, b); }
-    static __device__ __forceinline__ void split(F2 a, float& lo, float& hi) { f2split(a, lo, hi); }
-};
-template <> struct PairOf<double> {
-    using type = D2;
-    static __device__ __forceinline__ D2 make(double a, double b) { return D2{a, b}; }
-    static __device__ __forceinline__ D2 fma(D2 a, D2 b, D2 c) { return D2{::fma(a.lo, b.lo, c.lo), ::fma(a.hi, b.hi, c.hi)}; }
-    static __device__ __forceinline__ D2 mul(D2 a, D2 b) { return D2{__dmul_rn(a.lo, b.lo), __dmul_rn(a.hi, b.hi)}; }
-    static __device__ __forceinline__ void split(D2 a, double& lo, double& hi) {
-        lo = a.lo;
-        hi = a.hi;
-    }
-};
-
-// Per-object quantities of the column recursion.
-struct ShGeo {
-    double sinPhi, cosPhi, sinL, cosL, alpha, invCos;
-};
-// The per-object parts of the pair geopotential (shGeo, shDiagStart,
-// shDiagStep, shLowColumn and the column sums) are written with explicit
-// roundings (__fma_rn, __dmul_rn, ...): each lane evaluates them for both
-// objects of its pair, in two copies of the code, and an object's result must
-// not depend on whether it is the pair's first or second object (that is, on
-// which other object shares its warp).  Plain expressions would leave each
-// copy's multiply-add contraction to the compiler.
-static __device__ __forceinline__ ShGeo shGeo(double x, double y, double z, double R) {
-    ShGeo g;
-    const double rho2 = __fma_rn(y, y, __dmul_rn(x, x));
-    const double rn = __dsqrt_rn(__fma_rn(z, z, rho2));
-    const double rho = __dsqrt_rn(rho2);
-    g.sinPhi = __ddiv_rn(z, rn);
-    g.cosPhi = __ddiv_rn(rho, rn);
-    g.sinL = rho > 1e-14 ? __ddiv_rn(y, rho) : 0.0;
-    g.cosL = rho > 1e-14 ? __ddiv_rn(x, rho) : 1.0;
-    g.alpha = __ddiv_rn(R, rn);
-    g.invCos = g.cosPhi == 0.0 ? 0.0 : __drcp_rn(g.cosPhi);
-    return g;
-}
-
-// Diagonal of one object: P_mm, dP_mm, cos / sin m lambda, alpha^m, and the
-// closed-form step by W orders (P_{m+W} = D_m cos^W P_m, the phasor rotated
-// by W lambda, alpha^W), as shAccel forms them.
-struct ShDiag {
-    double Pmm, dPmm, cML, sML, am;
-    double cosW1, cLam, sLam, aW;  // cos^(W-1) phi, cos / sin W lambda, alpha^W
-};
-
-// FP64 low part of column `mcol` of one object (n = mcol .. lowDeg, tide
-// deltas for n <= 6): the six column sums and the FP32 start values of the
-// tile rows (degrees lowDeg + 1 and lowDeg).
-template <typename T, class Rec>
-static __device__ __forceinline__ void shLowColumn(const StepParams& p, const Rec& rec, const ShGeo& g,
-                                                   const ShDiag& d, int mcol, double S[6], T& P, T& P1, T& dP,
-                                                   T& dP1) {
-    const LowTable* __restrict__ low = p.low;
-    const int N = p.env.shDegree, lowDeg = p.lowDeg;
-    const bool tides = p.env.shTides != 0;
-    double Pn = d.Pmm, Pn1 = 0.0, dPn = d.dPmm, dPn1 = 0.0, an = d.am, anPrev = d.am;
-    const int nEnd = N < lowDeg ? N : lowDeg;
-    for (int k = 0; k < 6; ++k) S[k] = 0.0;
-    for (int n = mcol; n <= nEnd; ++n) {
-        const int ti = n * (n + 1) / 2 + mcol;
-        // order 0 has no sine term: nothing to read for it
-        double c = low->C[ti], s = mcol == 0 ? 0.0 : low->S[ti];
-        if (n <= 6 && tides) {
-            c = __dadd_rn(c, rec.dC(ti));
-            if (mcol != 0) s = __dadd_rn(s, rec.dS(ti));
-        }
-        const double q = __dmul_rn(an, Pn), qd = __dmul_rn(an, dPn), np1 = (double)(n + 1);
-        S[0] = __fma_rn(__dmul_rn(np1, c), q, S[0]);
-        S[1] = __fma_rn(__dmul_rn(np1, s), q, S[1]);
-        S[2] = __fma_rn(c, qd, S[2]);
-        S[3] = __fma_rn(s, qd, S[3]);
-        S[4] = __fma_rn(c, q, S[4]);
-        S[5] = __fma_rn(s, q, S[5]);
-        if (n < N) {
-            const int tn = (n + 1) * (n + 2) / 2 + mcol;
-            const double fa = low->a[tn], fb = low->b[tn];
-            const double P2 = Pn1;
-            Pn1 = Pn;
-            Pn = __fma_rn(__dmul_rn(fa, g.sinPhi), Pn1, -__dmul_rn(fb, P2));
-            const double dP2 = dPn1;
-            dPn1 = dPn;
-            dPn = __fma_rn(fa, __fma_rn(g.sinPhi, dPn1, __dmul_rn(g.cosPhi, Pn1)), -__dmul_rn(fb, dP2));
-            anPrev = an;
-            an = __dmul_rn(an, g.alpha);
-        }
-    }
-    P = (T)__dmul_rn(an, Pn);
-    P1 = (T)__dmul_rn(anPrev, Pn1);
-    dP = (T)__dmul_rn(an, dPn);
-    dP1 = (T)__dmul_rn(anPrev, dPn1);
-}
-
-static __device__ __forceinline__ void shDiagStart(const StepParams& p, const ShGeo& g, int first, int W,
-                                                   ShDiag& d) {
-    const double* __restrict__ diagC = p.diagC;
-    const int M = p.env.shOrder;
-    d.Pmm = 1.0;
-    d.dPmm = 0.0;
-    d.cML = 1.0;
-    d.sML = 0.0;
-    d.am = 1.0;
-    for (int m = 0; m < first && m < M; ++m) {
-        const double ns = __fma_rn(g.cosL, d.sML, __dmul_rn(g.sinL, d.cML));
-        const double nc = __fma_rn(g.cosL, d.cML, -__dmul_rn(g.sinL, d.sML));
-        d.sML = ns;
-        d.cML = nc;
-        const double cm = diagC[m + 1];
-        const double nP = __dmul_rn(__dmul_rn(cm, g.cosPhi), d.Pmm);
-        const double ndP = __dmul_rn(cm, __fma_rn(g.cosPhi, d.dPmm, -__dmul_rn(g.sinPhi, d.Pmm)));
-        d.Pmm = nP;
-        d.dPmm = ndP;
-        d.am = __dmul_rn(d.am, g.alpha);
-    }
-    d.cosW1 = 1.0;
-    d.cLam = 1.0;
-    d.sLam = 0.0;
-    d.aW = 1.0;
-    for (int t = 0; t < W - 1; ++t) d.cosW1 = __dmul_rn(d.cosW1, g.cosPhi);
-    for (int t = 0; t < W; ++t) {
-        const double ns = __fma_rn(g.cosL, d.sLam, __dmul_rn(g.sinL, d.cLam));
-        const double nc = __fma_rn(g.cosL, d.cLam, -__dmul_rn(g.sinL, d.sLam));
-        d.sLam = ns;
-        d.cLam = nc;
-        d.aW = __dmul_rn(d.aW, g.alpha);
-    }
-}
-
-// advance the diagonal from order m to m + W (shAccel's block step)
-static __device__ __forceinline__ void shDiagStep(const double2* __restrict__ diagStep, const ShGeo& g, int m, int W,
-                                                  ShDiag& d) {
-    const double2 f = diagStep[m];
-    const double cosWp = __dmul_rn(d.cosW1, g.cosPhi);
-    const double nP = __dmul_rn(__dmul_rn(f.x, cosWp), d.Pmm);
-    const double ndP = m == 0 ? __dmul_rn(__dmul_rn(__dmul_rn(-(double)W, g.sinPhi), d.cosW1), f.x)
-                              : __dmul_rn(__dmul_rn(f.y, cosWp), d.dPmm);
-    d.Pmm = nP;
-    d.dPmm = ndP;
-    const double ns = __fma_rn(d.cLam, d.sML, __dmul_rn(d.sLam, d.cML));
-    const double nc = __fma_rn(d.cLam, d.cML, -__dmul_rn(d.sLam, d.sML));
-    d.sML = ns;
-    d.cML = nc;
-    d.am = __dmul_rn(d.am, d.aW);
-}
-
-// one column's contribution (FP64 low sums S plus the tile part t) to an
-// object's (ar, aphi, alam) partial sums
-template <typename T>
-static __device__ __forceinline__ void columnSums(int mcol, const ShGeo& g, const ShDiag& d, const double S[6],
-                                                  const T t[6], double acc[3]) {
-    double c[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) c[k] = __dadd_rn(S[k], (double)t[k]);
-    const double mInv = __dmul_rn((double)mcol, g.invCos);
-    acc[0] = __dsub_rn(acc[0], __fma_rn(d.cML, c[0], __dmul_rn(d.sML, c[1])));
-    acc[1] = __dadd_rn(acc[1], __fma_rn(d.cML, c[2], __dmul_rn(d.sML, c[3])));
-    acc[2] = __dsub_rn(acc[2], __dmul_rn(mInv, __fma_rn(d.sML, c[4], -__dmul_rn(d.cML, c[5]))));
-}
-
-// Geopotential of the two objects of a pair of lane groups: the 2L lanes of
-// groups 2k and 2k+1 split the orders (lane pj of the pair takes
-// m = b 2L + pj, from the tile built for 2L lanes) and every lane runs its
-// columns for both objects (object of the first group, object of the
-// second), so each coefficient loaded from shared memory serves two objects
-// -- the column loop is bound by shared-memory bandwidth, not arithmetic.
-// Split precision runs the tile part as packed FP32 pairs (f32x2); FP64
-// runs it as two interleaved columns.  The low part and the diagonal stay
-// FP64 per object.  Returns the calling lane's own object's acceleration
-// (body frame, km/s^2), the same on every lane of its group.
-template <int L, typename T, class Rec>
-static __device__ __forceinline__ void shAccelPair(const StepParams& p, const typename TileOf<T>::type* __restrict__ tile,
-                                                   const Rec& rec, double x, double y, double z, double out[3]) {
-    using Pr = PairOf<T>;
-    using V = typename Pr::type;
-    using Tile = typename TileOf<T>::type;
-    constexpr int W = 2 * L;
-    const int lane = (int)(threadIdx.x & 31);
-    const int pj = lane % W;
-    const bool second = pj >= L;
-    const unsigned pairMask = W >= 32 ? 0xffffffffu : (((1u << W) - 1u) << (lane - pj));
-    const int N = p.env.shDegree, M = p.env.shOrder;
-    const int lowDeg = p.lowDeg;
-    const double ox = __shfl_xor_sync(pairMask, x, L), oy = __shfl_xor_sync(pairMask, y, L),
-                 oz = __shfl_xor_sync(pairMask, z, L);
-    const Rec orec = rec.partner(pairMask, L);
-    const ShGeo g0 = second ? shGeo(ox, oy, oz, p.env.shR) : shGeo(x, y, z, p.env.shR);
-    const ShGeo g1 = second ? shGeo(x, y, z, p.env.shR) : shGeo(ox, oy, oz, p.env.shR);
-    const Rec& r0 = second ? orec : rec;
-    const Rec& r1 = second ? rec : orec;
-    ShDiag d0, d1;
-    shDiagStart(p, g0, pj, W, d0);
-    shDiagStart(p, g1, pj, W, d1);
-    const V u = Pr::make((T)(g0.alpha * g0.sinPhi), (T)(g1.alpha * g1.sinPhi));
-    const V v = Pr::make((T)(g0.alpha * g0.cosPhi), (T)(g1.alpha * g1.cosPhi));
-    const V a2 = Pr::make((T)(g0.alpha * g0.alpha), (T)(g1.alpha * g1.alpha));
-    double acc0[3] = {0.0, 0.0, 0.0}, acc1[3] = {0.0, 0.0, 0.0};  // ar, aphi, alam
-    const double2* __restrict__ diagStep = p.diagStep;
-    const int nblocks = p.nblocks;
-    for (int b = 0; b < nblocks; ++b) {
-        const int mcol = b * W + pj;
-        const bool act = mcol <= M;
-        double S0[6] = {0, 0, 0, 0, 0, 0}, S1[6] = {0, 0, 0, 0, 0, 0};
-        T P0 = T(0), P10 = T(0), dP0 = T(0), dP10 = T(0), P1_ = T(0), P11 = T(0), dP1_ = T(0), dP11 = T(0);
-        if (act && mcol <= lowDeg) {
-            shLowColumn<T>(p, r0, g0, d0, mcol, S0, P0, P10, dP0, dP10);
-            shLowColumn<T>(p, r1, g1, d1, mcol, S1, P1_, P11, dP1_, dP11);
-        } else if (act) {
-            P0 = (T)(d0.am * d0.Pmm);
-            dP0 = (T)(d0.am * d0.dPmm);
-            P1_ = (T)(d1.am * d1.Pmm);
-            dP1_ = (T)(d1.am * d1.dPmm);
-        }
-        V P = Pr::make(P0, P1_), Pm1 = Pr::make(P10, P11), dP = Pr::make(dP0, dP1_), dPm1 = Pr::make(dP10, dP11);
-        V Scc = Pr::make(T(0), T(0)), Ssc = Scc, Spc = Scc, Sps = Scc, Sdc = Scc, Sds = Scc;
-        const int2 blk = p.blocks[b];
-        const Tile* tp = tile + blk.x + pj;
-        for (int i = 0; i < blk.y; ++i, tp += W) {
-            const Tile e = *tp;
-            const V c = Pr::make(T(e.c), T(e.c)), s = Pr::make(T(e.s), T(e.s));
-            const V cp = Pr::make(T(e.cp), T(e.cp)), sp = Pr::make(T(e.sp), T(e.sp));
-            const V fa = Pr::make(T(e.a), T(e.a)), nb = Pr::make(-T(e.b), -T(e.b));
-            Scc = Pr::fma(cp, P, Scc);
-            Ssc = Pr::fma(sp, P, Ssc);
-            Spc = Pr::fma(c, P, Spc);
-            Sps = Pr::fma(s, P, Sps);
-            Sdc = Pr::fma(c, dP, Sdc);
-            Sds = Pr::fma(s, dP, Sds);
-            const V Pn = Pr::fma(fa, Pr::mul(u, P), Pr::mul(nb, Pr::mul(a2, Pm1)));
-            const V dPn = Pr::fma(fa, Pr::fma(u, dP, Pr::mul(v, P)), Pr::mul(nb, Pr::mul(a2, dPm1)));
-            Pm1 = P;
-            P = Pn;
-            dPm1 = dP;
-            dP = dPn;
-        }
-        if (act) {
-            T t0[6], t1[6];
-            Pr::split(Scc, t0[0], t1[0]);
-            Pr::split(Ssc, t0[1], t1[1]);
-            Pr::split(Sdc, t0[2], t1[2]);
-            Pr::split(Sds, t0[3], t1[3]);
-            Pr::split(Spc, t0[4], t1[4]);
-            Pr::split(Sps, t0[5], t1[5]);
-            columnSums<T>(mcol, g0, d0, S0, t0, acc0);
-            columnSums<T>(mcol, g1, d1, S1, t1, acc1);
-        }
-        const int m = b * W + pj;
-        if (m + W <= M) {
-            shDiagStep(diagStep, g0, m, W, d0);
-            shDiagStep(diagStep, g1, m, W, d1);
-        }
-    }
-    // fold the pair's lanes: both objects' partial sums over all 2L lanes
-#pragma unroll
-    for (int off = W / 2; off > 0; off >>= 1)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            acc0[k] += __shfl_xor_sync(pairMask, acc0[k], off);
-            acc1[k] += __shfl_xor_sync(pairMask, acc1[k], off);
-        }
-    const ShGeo& g = second ? g1 : g0;
-    double ar = second ? acc1[0] : acc0[0], aphi = second ? acc1[1] : acc0[1], alam = second ? acc1[2] : acc0[2];
-    if (g.cosPhi == 0.0 && M >= 1) {
-        // exact pole: the m = 1 longitudinal term's analytical limit (as shAccel)
-        const bool tides = p.env.shTides != 0;
-        double an = g.alpha;
-        for (int n = 1; n <= N; ++n) {
-            const int ti = n * (n + 1) / 2 + 1;
-            double s = p.env.shS[ti];
-            if (n <= 6 && tides) s += rec.dS(ti);
-            const double sign = g.sinPhi > 0.0 ? 1.0 : ((n & 1) ? 1.0 : -1.0);
-            double lim = 0.5 * (double)n * (n + 1.0);
-            if (p.env.shNormalized) lim *= sqrt(2.0 * (2.0 * n + 1.0) / ((double)n * (n + 1.0)));
-            alam -= an * (sign * lim) * (-s);
-            an *= g.alpha;
-        }
-    }
-    (void)lowDeg;
-    const double rn = p.env.shR / g.alpha;
-    const double gm = p.env.shGM / (rn * rn);
-    ar *= gm;
-    aphi *= gm;
-    alam *= gm;
-    out[0] = g.cosPhi * g.cosL * ar - g.sinPhi * g.cosL * aphi - g.sinL * alam;
-    out[1] = g.cosPhi * g.sinL * ar - g.sinPhi * g.sinL * aphi + g.cosL * alam;
-    out[2] = g.sinPhi * ar + g.cosPhi * aphi;
 }
 
 // ---- the remaining forces ------------------------------------------------------------------
@@ -891,10 +369,10 @@ static __device__ __noinline__ void tideAloneAccel(const Rec r, const double pos
 }
 
 // full right-hand side acceleration (km/s^2); every lane of the group calls it.
-// PAIR: the geopotential of lane-group pairs (a separate kernel instantiation,
+// PAIR: two lane groups share their columns (a separate kernel instantiation,
 // so the one-object-per-lane kernel keeps its own register allocation).
 template <int L, typename T, bool PAIR, class Rec>
-static __device__ __forceinline__ void accelerations(const StepParams& p, const typename TileOf<T>::type* tile,
+static __device__ __forceinline__ void accelerations(const StepParams& p, const void* tile,
                                               const Rec& r, const double pos[3], const double vel[3],
                                               double bc, double ams, double acc[3]) {
     const DevEnv& e = p.env;
@@ -942,21 +420,13 @@ static __device__ __forceinline__ void accelerations(const StepParams& p, const 
                 bz = r.SR(6) * d0 + r.SR(7) * d1 + r.SR(8) * d2;
             }
             double a[3];
-            if constexpr (!std::is_same<T, double>::value) {
-                // split precision: objects below the split radius keep the
-                // tile part in FP64 (from the FP64 tile in global memory)
-                if constexpr (PAIR)
-                    shAccelPair<L, T>(p, tile, r, bx, by, bz, a);
-                else if (p.splitRadius > 0.0 && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius)
-                    shAccel<L, double>(p, (const TileD*)p.tile64, r, bx, by, bz, a);
-                else
-                    shAccel<L, T>(p, tile, r, bx, by, bz, a);
-            } else {
-                if constexpr (PAIR)
-                    shAccelPair<L, T>(p, tile, r, bx, by, bz, a);
-                else
-                    shAccel<L, T>(p, tile, r, bx, by, bz, a);
-            }
+            // split precision with a floor: objects below the split radius
+            // keep every row in FP64 (from the FP64 tile in global memory)
+            if (!PAIR && sizeof(T) == 4 && p.splitRadius > 0.0
+                && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius)
+                fieldAccel<L, 1, double>(p, p.tile64, p.blocks64, p.nblocks64, r, bx, by, bz, a);
+            else
+                fieldAccel<L, PAIR ? 2 : 1, T>(p, tile, p.blocks, p.nblocks, r, bx, by, bz, a);
             double ai[3];
             if (isEarth) {
                 fromBody(r, a, ai);
@@ -1180,10 +650,9 @@ static __device__ __forceinline__ RecordInterp recordFromGrid(const StepParams& 
 // 320 or 384 threads leave 168 registers a thread and 256 threads leave 255).
 template <int L, typename T, bool SHARED_GRID, bool PAIR, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant__ StepParams p) {
-    using Tile = typename TileOf<T>::type;
     constexpr int CPL = (6 + L - 1) / L;
     extern __shared__ __align__(128) unsigned char smem[];
-    const Tile* tile = (const Tile*)p.tile;
+    const void* tile = p.tile;
     int kOffset = 0;
     if (!SHARED_GRID && !p.gridPairs) {  // per-object time needs the batch's record grid
         if (threadIdx.x == 0) atomicExch(p.errorFlag, 3);
@@ -1192,7 +661,7 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
     if (p.useSmemTile) {
         const bool test = p.tileWaitTest != 0;
         if (stageTile(smem, p.tile, p.tileBytes, !test, test ? 4096L : (1L << 24)))
-            tile = (const Tile*)smem;
+            tile = smem;
         else if (threadIdx.x == 0 && p.tileFallbacks)
             atomicAdd(p.tileFallbacks, 1);  // this CTA reads the tile from global memory
         kOffset = p.tileBytes;

@@ -280,8 +280,6 @@ int Server::step() {
         p.state = state_;
         p.bc = bc_;
         p.ams = ams_;
-        p.low = engine_.dLow_;
-        p.diagC = engine_.dDiag_;
         p.maxSteps = K;
         p.order = order;
         p.cur = cur_;
