@@ -1517,7 +1517,7 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
         p.splitRadius = host_.shR + opt.splitFloorKm;
     }
     // shared memory per CTA: the coefficient tile (when it fits) plus the
-    // stage derivatives, 13 x ceil(6/L) doubles per thread
+    // stage accelerations of its objects
     int registers = 0;
     int threadsReq = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs));
     {
@@ -1533,14 +1533,14 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
         threadsReq = std::max(32, std::min(threadsReq, at->second.first / 32 * 32));
         registers = at->second.second;
     }
-    const int kPerThread = 13 * ((6 + L - 1) / L) * 8;
     int threads = threadsReq;
-    if (opt.tileSmem != 0 && tile.bytes + 1024 + 64 * kPerThread <= maxSmem_) {
+    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - bytes) / kStageBytes * L / 32 * 32; };
+    if (opt.tileSmem != 0 && tile.bytes + 1024 <= maxSmem_ && fit(tile.bytes) >= 64) {
         p.useSmemTile = 1;
-        threads = std::min(threadsReq, (maxSmem_ - tile.bytes - 1024) / kPerThread / 32 * 32);
+        threads = std::min(threadsReq, fit(tile.bytes));
     } else {
         p.useSmemTile = 0;
-        threads = std::min(threadsReq, (maxSmem_ - 1024) / kPerThread / 32 * 32);
+        threads = std::min(threadsReq, fit(0));
     }
     int perSm = opt.ctasPerSm;
     if (perSm <= 0) {

@@ -205,15 +205,10 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.workCounter = ctl;
     sp.errorFlag = ctl + 1;
     const int threadsReq = std::min(opt.threads > 0 ? opt.threads : 512, maxStepThreads(L));
-    const int kPerThread = 13 * ((6 + L - 1) / L) * 8;
-    int threads;
-    if (opt.tileSmem != 0 && (int)ht.bytes.size() + 1024 + 64 * kPerThread <= maxSmem_) {
-        sp.useSmemTile = 1;
-        threads = std::min(threadsReq, (maxSmem_ - (int)ht.bytes.size() - 1024) / kPerThread / 32 * 32);
-    } else {
-        sp.useSmemTile = 0;
-        threads = std::min(threadsReq, (maxSmem_ - 1024) / kPerThread / 32 * 32);
-    }
+    const int tileBytes = (int)ht.bytes.size();
+    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - bytes) / kStageBytes * L / 32 * 32; };
+    sp.useSmemTile = opt.tileSmem != 0 && tileBytes + 1024 <= maxSmem_ && fit(tileBytes) >= 64;
+    const int threads = std::min(threadsReq, fit(sp.useSmemTile ? tileBytes : 0));
     const int smem = propagateSmemBytes(sp, L, threads);
     int perSm = opt.ctasPerSm > 0 ? opt.ctasPerSm : propagateMaxCtasPerSm(L, opt.split, true, 0, 0, threads, smem);
     if (perSm <= 0) perSm = 1;

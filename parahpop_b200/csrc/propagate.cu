@@ -85,8 +85,7 @@ void launchRecordPairs(const EpochRecord* grid, int64_t count, double2* pairs, c
 }
 
 int propagateSmemBytes(const StepParams& p, int lanes, int threads) {
-    const int cpl = (6 + lanes - 1) / lanes;
-    return (p.useSmemTile ? p.tileBytes : 0) + 13 * cpl * threads * (int)sizeof(double);
+    return (p.useSmemTile ? p.tileBytes : 0) + kStageBytes * (threads / lanes);
 }
 
 int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int threads, int smem) {

@@ -7,12 +7,11 @@
 //
 // Work split (autotuned):  L lanes (1, 2, 4, 8 or 16) cooperate on one object,
 // a warp holds 32/L objects.
-//   * RK state: lane j of a group owns the state components d with d % L == j,
-//     keeps y_d in registers and the 13 stage derivatives k_s[d] in shared
-//     memory ([stage][component][thread], conflict-free), forms the
-//     stage state for its components in the reference's order
-//     (parm/integrate/rk/host/Step.h:33-84) and the 8th-order update in stage
-//     order (Step.h:86-104), and broadcasts components by warp shuffle.
+//   * RK state: a lane of a group owns coordinate axes (position and velocity
+//     in registers); the stage accelerations lie in shared memory, from which
+//     the lane forms its axes' stage state (the reference's sums,
+//     parm/integrate/rk/host/Step.h:33-104, with the position rows summed on
+//     accelerations) and broadcasts it by warp shuffle.
 //   * Spherical harmonics: the field's acceleration as column sums of solid
 //     harmonics one degree up (geopotential.hpp), orders M in blocks of L
 //     columns (2L where two lane groups share their columns: every lane then
@@ -104,6 +103,9 @@ struct StepParams {
     int* errorFlag;
     int* tileFallbacks;     // CTAs whose tile staging timed out (read the tile from global memory); nullable
 };
+
+// shared memory of one object's stage accelerations: ten slots of three doubles
+constexpr int kStageBytes = 10 * 3 * 8;
 
 // Threads per CTA the step kernel is compiled for: narrow lane splits run one
 // CTA of few threads per SM (the coefficient tile fills shared memory), so

@@ -46,65 +46,115 @@ __host__ __device__ constexpr double rkB(int s) {
          : s == 11 ? 41. / 840 : s == 12 ? 41. / 840 : 0;
 }
 
-// ---- RK stage storage ------------------------------------------------------------------------
-// Lane j of a group owns state components d = j + c*L (c < CPL).  The stage
-// derivatives live in shared memory, [stage][component slot][thread], so that
-// consecutive threads hit consecutive banks.
-static __constant__ double c_rkA[12][12] = {
-    {2. / 27, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0},
-    {1. / 36, 1. / 12, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0},
-    {1. / 24, 0, 1. / 8, 0, 0, 0, 0, 0, 0, 0, 0, 0},
-    {5. / 12, 0, -25. / 16, 25. / 16, 0, 0, 0, 0, 0, 0, 0, 0},
-    {1. / 20, 0, 0, 1. / 4, 1. / 5, 0, 0, 0, 0, 0, 0, 0},
-    {-25. / 108, 0, 0, 125. / 108, -65. / 27, 125. / 54, 0, 0, 0, 0, 0, 0},
-    {31. / 300, 0, 0, 0, 61. / 225, -2. / 9, 13. / 900, 0, 0, 0, 0, 0},
-    {2.0, 0, 0, -53. / 6, 704. / 45, -107. / 9, 67. / 90, 3.0, 0, 0, 0, 0},
-    {-91. / 108, 0, 0, 23. / 108, -976. / 135, 311. / 54, -19. / 60, 17. / 6, -1. / 12, 0, 0, 0},
-    {2383. / 4100, 0, 0, -341. / 164, 4496. / 1025, -301. / 82, 2133. / 4100, 45. / 82, 45. / 164, 18. / 41, 0, 0},
-    {3. / 205, 0, 0, 0, 0, -6. / 41, -3. / 205, -3. / 41, 3. / 41, 6. / 41, 0, 0},
-    {-1777. / 4100, 0, 0, -341. / 164, 4496. / 1025, -289. / 82, 2193. / 4100, 51. / 82, 33. / 164, 12. / 41, 0, 1.0}};
+// ---- RK stages on accelerations alone -------------------------------------------------------
+// The right-hand side is y'' = f(t, y, y'), so the position rows of the stage
+// sums are sums of the velocity rows' own sums: with k_j the accelerations,
+//     v_s = v + dt sum_j a_sj k_j
+//     y_s = y + dt c_s v + dt^2 sum_j (A A)_sj k_j
+// and the same for the update with b and b A.  Only accelerations are kept:
+// ten slots of three doubles an object, against thirteen stages of six
+// components.  Stage 10 (c = 1) enters neither another stage nor the
+// 8th-order update (it serves the 7th-order error estimate, which a fixed
+// step does not form), so it is not evaluated; stage 11 takes the slot of
+// stage 1, whose last reader is stage 4.  rkAA and rkBA are the exact
+// rational products.  At one lane per object the 624 bytes of stage
+// derivatives an object left 128 threads a CTA beside the degree-70 tile; 240
+// bytes leave room for all 256: 200,000 uneven objects x 8 steps FP64 86.6 ->
+// 66.3 ms, 10^6 x 4 split 126 -> 110 ms, 10^4 LEO x 20 FP64 16.2 -> 14.9 ms.
+__host__ __device__ constexpr double rkAA(int s, int j) {
+    return s == 2 ? (j == 0 ? 1. / 162 : 0)
+         : s == 3 ? (j == 0 ? 1. / 288 : j == 1 ? 1. / 96 : 0)
+         : s == 4 ? (j == 0 ? 25. / 1152 : j == 1 ? -25. / 192 : j == 2 ? 25. / 128 : 0)
+         : s == 5 ? (j == 0 ? 3. / 32 : j == 2 ? -9. / 32 : j == 3 ? 5. / 16 : 0)
+         : s == 6 ? (j == 0 ? -725. / 864 : j == 2 ? 125. / 32 : j == 3 ? -1375. / 432 : j == 4 ? 25. / 54 : 0)
+         : s == 7 ? (j == 0 ? 383. / 3888 : j == 2 ? -61. / 144 : j == 3 ? 187. / 486 : j == 4 ? -77. / 972
+                    : j == 5 ? 65. / 1944 : 0)
+         : s == 8 ? (j == 0 ? 553427. / 97200 : j == 2 ? -3679. / 144 : j == 3 ? 43417. / 1944
+                    : j == 4 ? -40783. / 12150 : j == 5 ? 1027. / 972 : j == 6 ? 13. / 300 : 0)
+         : s == 9 ? (j == 0 ? -163043. / 64800 : j == 2 ? 1087. / 96 : j == 3 ? -12295. / 1296
+                    : j == 4 ? 11167. / 8100 : j == 5 ? -241. / 648 : j == 6 ? -19. / 900 : j == 7 ? -1. / 4 : 0)
+         : s == 11 ? (j == 0 ? 71. / 6150 : j == 3 ? -329. / 492 : j == 4 ? 224. / 3075 : j == 5 ? -11. / 246
+                     : j == 6 ? 29. / 4100 : j == 7 ? 26. / 41 : j == 8 ? -1. / 82 : 0)
+         : s == 12 ? (j == 0 ? 54963. / 32800 : j == 2 ? -9333. / 1312 : j == 3 ? 3199. / 656
+                     : j == 4 ? -3247. / 4100 : j == 5 ? 81. / 328 : j == 6 ? 211. / 4100 : j == 7 ? 223. / 164
+                     : j == 8 ? 2. / 41 : j == 9 ? 6. / 41 : 0)
+         : 0;
+}
+__host__ __device__ constexpr double rkBA(int j) {
+    return j == 5 ? 17. / 105 : j == 6 ? 3. / 70 : j == 7 ? 3. / 14 : j == 8 ? 3. / 280 : j == 9 ? 3. / 140
+         : j == 11 ? 41. / 840 : 0;
+}
+__host__ __device__ constexpr int rkSlot(int s) { return s == 11 ? 1 : s; }
 
-template <int CPL>
-struct StageStore {
-    double* base;  // shared memory, 13 * CPL * blockDim doubles
-    int stride;    // blockDim.x
-    __device__ __forceinline__ double& at(int s, int c) const {
-        return base[((s * CPL) + c) * stride + threadIdx.x];
+// A lane owns AXES coordinate axes (position and velocity): all three at one
+// lane per object; axes j and 2 at two lanes (both lanes carry axis 2); axis
+// j % 3 at four and more.  The accelerations of the stages lie in shared
+// memory, [slot][axis][object of the CTA].
+template <int L>
+struct Axes {
+    static constexpr int N = L == 1 ? 3 : L == 2 ? 2 : 1;
+    static __device__ __forceinline__ int axis(int j, int i) {
+        return L == 1 ? i : L == 2 ? (i == 0 ? j : 2) : j % 3;
     }
+    // the lane that writes axis(j, i) to memory
+    static __device__ __forceinline__ bool writes(int j, int i) {
+        return L == 1 ? true : L == 2 ? (i == 0 || j == 0) : j < 3;
+    }
+    // lane and place of axis a
+    static __host__ __device__ constexpr int lane(int a) { return L == 1 ? 0 : L == 2 ? (a == 2 ? 0 : a) : a; }
+    static __host__ __device__ constexpr int place(int a) { return L == 1 ? a : L == 2 ? (a == 2 ? 1 : 0) : 0; }
 };
 
-// y_s = y + sum_j (dt a_sj) k_j in stage order (Step.h:33-84)
-template <int CPL>
-static __device__ __forceinline__ void combine(int s, const double (&y)[CPL], const StageStore<CPL>& k, double dt,
-                                        double (&ys)[CPL]) {
+struct StageStore {
+    double* base;  // this object's first slot
+    int stride;    // objects of the CTA
+    __device__ __forceinline__ double& at(int slot, int axis) const { return base[(slot * 3 + axis) * stride]; }
+};
+
+// position and velocity of the lane's axes at stage S
+template <int L, int S>
+static __device__ __forceinline__ void stageState(const double (&y)[Axes<L>::N], const double (&v)[Axes<L>::N],
+                                                  const StageStore& k, int j, double dt, double (&ys)[Axes<L>::N],
+                                                  double (&vs)[Axes<L>::N]) {
+    const double dt2 = dt * dt;
 #pragma unroll
-    for (int c = 0; c < CPL; ++c) ys[c] = y[c];
-    for (int jj = 0; jj < s; ++jj) {
-        const double a = c_rkA[s - 1][jj];
-        if (a != 0.0) {
-            const double coef = dt * a;
+    for (int i = 0; i < Axes<L>::N; ++i) {
+        const int axis = Axes<L>::axis(j, i);
+        double sv = 0.0, sy = 0.0;
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) ys[c] = fma(coef, k.at(jj, c), ys[c]);
+        for (int l = 0; l < S; ++l) {
+            if (rkA(S - 1, l) != 0.0 || rkAA(S, l) != 0.0) {
+                const double kl = k.at(rkSlot(l), axis);
+                if (rkA(S - 1, l) != 0.0) sv = fma(rkA(S - 1, l), kl, sv);
+                if (rkAA(S, l) != 0.0) sy = fma(rkAA(S, l), kl, sy);
+            }
         }
+        ys[i] = fma(dt2, sy, fma(dt * rkC(S - 1), v[i], y[i]));
+        vs[i] = fma(dt, sv, v[i]);
     }
 }
 
-// y += sum_s (dt b_s) k_s in stage order (Step.h:86-104)
-template <int CPL>
-static __device__ __forceinline__ void finalUpdate(double (&y)[CPL], const StageStore<CPL>& k, double dt, bool apply) {
-    double yn[CPL];
+// the 8th-order update of the lane's axes; acc is stage 12's acceleration
+template <int L>
+static __device__ __forceinline__ void finalUpdate(double (&y)[Axes<L>::N], double (&v)[Axes<L>::N],
+                                                   const StageStore& k, int j, double dt, const double acc[3],
+                                                   bool apply) {
 #pragma unroll
-    for (int c = 0; c < CPL; ++c) yn[c] = y[c];
+    for (int i = 0; i < Axes<L>::N; ++i) {
+        const int axis = Axes<L>::axis(j, i);
+        double sv = 0.0, sy = 0.0;
 #pragma unroll
-    for (int s = 0; s < 13; ++s)
-        if (rkB(s) != 0.0) {
-            const double cb = dt * rkB(s);
-#pragma unroll
-            for (int c = 0; c < CPL; ++c) yn[c] = fma(cb, k.at(s, c), yn[c]);
+        for (int l = 5; l < 12; ++l)
+            if (rkB(l) != 0.0) {
+                const double kl = k.at(rkSlot(l), axis);
+                sv = fma(rkB(l), kl, sv);
+                sy = fma(rkBA(l), kl, sy);
+            }
+        sv = fma(rkB(12), axis == 0 ? acc[0] : axis == 1 ? acc[1] : acc[2], sv);
+        if (apply) {
+            y[i] = fma(dt, fma(dt, sy, v[i]), y[i]);
+            v[i] = fma(dt, sv, v[i]);
         }
-    if (apply) {
-#pragma unroll
-        for (int c = 0; c < CPL; ++c) y[c] = yn[c];
     }
 }
 
@@ -650,7 +700,7 @@ static __device__ __forceinline__ RecordInterp recordFromGrid(const StepParams& 
 // 320 or 384 threads leave 168 registers a thread and 256 threads leave 255).
 template <int L, typename T, bool SHARED_GRID, bool PAIR, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant__ StepParams p) {
-    constexpr int CPL = (6 + L - 1) / L;
+    constexpr int NA = Axes<L>::N;
     extern __shared__ __align__(128) unsigned char smem[];
     const void* tile = p.tile;
     int kOffset = 0;
@@ -666,7 +716,7 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
             atomicAdd(p.tileFallbacks, 1);  // this CTA reads the tile from global memory
         kOffset = p.tileBytes;
     }
-    StageStore<CPL> kst{(double*)(smem + kOffset), (int)blockDim.x};
+    const StageStore kst{(double*)(smem + kOffset) + threadIdx.x / L, (int)blockDim.x / L};
     const int lane = (int)(threadIdx.x & 31);
     const int j = lane % L;
     const int g = lane / L;
@@ -691,11 +741,12 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
         const int64_t sidx = valid ? slot : p.n - 1;
         const int64_t oi = p.order ? p.order[sidx] : sidx;
         const int64_t stride = p.stride ? p.stride : p.n;
-        double y[CPL];
+        double y[NA], v[NA];
 #pragma unroll
-        for (int c = 0; c < CPL; ++c) {
-            const int d = j + c * L;
-            y[c] = d < 6 ? p.state[(int64_t)d * stride + oi] : 0.0;
+        for (int i = 0; i < NA; ++i) {
+            const int axis = Axes<L>::axis(j, i);
+            y[i] = p.state[(int64_t)axis * stride + oi];
+            v[i] = p.state[(int64_t)(axis + 3) * stride + oi];
         }
         const double bc = p.bc[oi], ams = p.ams[oi];
         double cur = 0.0, dtv = 0.0, endv = 0.0, stepv = 0.0;
@@ -714,18 +765,39 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
             }
             const double t0 = SHARED_GRID ? p.stepT0[kstep] : cur;
             const double dt = SHARED_GRID ? p.stepDt[kstep] : dtv;
+            double acc[3];
             // one copy of the force model: the stage loop is not unrolled
 #pragma unroll 1
             for (int s = 0; s < 13; ++s) {
-                double ys[CPL];
-                combine<CPL>(s, y, kst, dt, ys);
+                double ys[NA], vs[NA];
+                switch (s) {
+                    case 0:
+#pragma unroll
+                        for (int i = 0; i < NA; ++i) {
+                            ys[i] = y[i];
+                            vs[i] = v[i];
+                        }
+                        break;
+                    case 1: stageState<L, 1>(y, v, kst, j, dt, ys, vs); break;
+                    case 2: stageState<L, 2>(y, v, kst, j, dt, ys, vs); break;
+                    case 3: stageState<L, 3>(y, v, kst, j, dt, ys, vs); break;
+                    case 4: stageState<L, 4>(y, v, kst, j, dt, ys, vs); break;
+                    case 5: stageState<L, 5>(y, v, kst, j, dt, ys, vs); break;
+                    case 6: stageState<L, 6>(y, v, kst, j, dt, ys, vs); break;
+                    case 7: stageState<L, 7>(y, v, kst, j, dt, ys, vs); break;
+                    case 8: stageState<L, 8>(y, v, kst, j, dt, ys, vs); break;
+                    case 9: stageState<L, 9>(y, v, kst, j, dt, ys, vs); break;
+                    case 10: continue;  // enters neither a stage nor the update
+                    case 11: stageState<L, 11>(y, v, kst, j, dt, ys, vs); break;
+                    default: stageState<L, 12>(y, v, kst, j, dt, ys, vs); break;
+                }
                 double st[6];
 #pragma unroll
-                for (int d = 0; d < 6; ++d) {
-                    const double own = ys[(d / L) < CPL ? (d / L) : 0];
-                    st[d] = (L == 1) ? ys[d < CPL ? d : 0] : __shfl_sync(0xffffffffu, own, groupBase + d % L);
+                for (int a = 0; a < 3; ++a) {
+                    const double py = ys[Axes<L>::place(a)], pv = vs[Axes<L>::place(a)];
+                    st[a] = L == 1 ? py : __shfl_sync(0xffffffffu, py, groupBase + Axes<L>::lane(a));
+                    st[a + 3] = L == 1 ? pv : __shfl_sync(0xffffffffu, pv, groupBase + Axes<L>::lane(a));
                 }
-                double acc[3];
                 if (SHARED_GRID) {
                     const RecordRef rec{p.records + kstep * 13 + s};
                     accelerations<L, T, PAIR>(p, tile, rec, st, st + 3, bc, ams, acc);
@@ -734,20 +806,28 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
                     const RecordInterp rec = recordFromGrid(p, ts);
                     accelerations<L, T, PAIR>(p, tile, rec, st, st + 3, bc, ams, acc);
                 }
+                if (s < 12) {
 #pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    const int d = j + c * L;
-                    kst.at(s, c) = d < 3 ? st[d + 3] : (d < 6 ? acc[d - 3] : 0.0);
+                    for (int i = 0; i < NA; ++i) {
+                        const int axis = Axes<L>::axis(j, i);
+                        if (Axes<L>::writes(j, i))
+                            kst.at(rkSlot(s), axis) = axis == 0 ? acc[0] : axis == 1 ? acc[1] : acc[2];
+                    }
+                    if (L > 1) __syncwarp();
                 }
             }
-            finalUpdate<CPL>(y, kst, dt, SHARED_GRID || !done);
+            finalUpdate<L>(y, v, kst, j, dt, acc, SHARED_GRID || !done);
+            if (L > 1) __syncwarp();
             if (SHARED_GRID && p.traj && (kstep + 1) % p.trajEvery == 0 && valid
                 && (kstep + 1) / p.trajEvery <= p.trajRecords) {
                 double* rec = p.traj + (int64_t)((kstep + 1) / p.trajEvery - 1) * 6 * p.n;
 #pragma unroll
-                for (int c = 0; c < CPL; ++c) {
-                    const int d = j + c * L;
-                    if (d < 6) rec[(int64_t)d * p.n + oi] = y[c];
+                for (int i = 0; i < NA; ++i) {
+                    const int axis = Axes<L>::axis(j, i);
+                    if (Axes<L>::writes(j, i)) {
+                        rec[(int64_t)axis * p.n + oi] = y[i];
+                        rec[(int64_t)(axis + 3) * p.n + oi] = v[i];
+                    }
                 }
             }
             if (!SHARED_GRID && !done) {
@@ -760,9 +840,12 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
         }
         if (valid) {
 #pragma unroll
-            for (int c = 0; c < CPL; ++c) {
-                const int d = j + c * L;
-                if (d < 6) p.state[(int64_t)d * stride + oi] = y[c];
+            for (int i = 0; i < NA; ++i) {
+                const int axis = Axes<L>::axis(j, i);
+                if (Axes<L>::writes(j, i)) {
+                    p.state[(int64_t)axis * stride + oi] = y[i];
+                    p.state[(int64_t)(axis + 3) * stride + oi] = v[i];
+                }
             }
             if (!SHARED_GRID && j == 0) {
                 p.cur[oi] = cur;
