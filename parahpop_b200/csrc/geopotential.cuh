@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "geopotential.hpp"
 #include "propagate.cuh"
 
@@ -114,28 +116,57 @@ static __device__ __forceinline__ void fieldRow(T a, T xc, T xs, T yc, T ys, T z
     q = n;
 }
 
-// `pairs` FP64 row pairs of one column, W lanes interleaved
+// The tile, in global memory or staged at the start of the CTA's dynamic
+// shared memory.
+extern __shared__ __align__(128) unsigned char g_smem[];
+struct TileRef {
+    const void* global;
+    bool staged;
+};
+
+// One row pair of a column, W lanes interleaved.
 template <int K, int W>
-static __device__ __forceinline__ void fieldRows(const double2* __restrict__ tp, int pairs, const Lanes<double, K>& u,
-                                                 const Lanes<double, K>& t, Lanes<double, K>& q, Lanes<double, K>& q1,
-                                                 Lanes<double, K> (&S)[6]) {
-    for (int i = 0; i < pairs; ++i, tp += kChunks64 * W) {
-        const double2 a = tp[0], x0 = tp[W], y0 = tp[2 * W], z0 = tp[3 * W];
-        const double2 x1 = tp[4 * W], y1 = tp[5 * W], z1 = tp[6 * W];
-        fieldRow<double, K>(a.x, x0.x, x0.y, y0.x, y0.y, z0.x, z0.y, u, t, q, q1, S);
-        fieldRow<double, K>(a.y, x1.x, x1.y, y1.x, y1.y, z1.x, z1.y, u, t, q, q1, S);
-    }
+static __device__ __forceinline__ void rowPair(const double2* __restrict__ tp, const Lanes<double, K>& u,
+                                               const Lanes<double, K>& t, Lanes<double, K>& q, Lanes<double, K>& q1,
+                                               Lanes<double, K> (&S)[6]) {
+    const double2 a = tp[0], x0 = tp[W], y0 = tp[2 * W], z0 = tp[3 * W];
+    const double2 x1 = tp[4 * W], y1 = tp[5 * W], z1 = tp[6 * W];
+    fieldRow<double, K>(a.x, x0.x, x0.y, y0.x, y0.y, z0.x, z0.y, u, t, q, q1, S);
+    fieldRow<double, K>(a.y, x1.x, x1.y, y1.x, y1.y, z1.x, z1.y, u, t, q, q1, S);
 }
 template <int K, int W>
-static __device__ __forceinline__ void fieldRows(const float4* __restrict__ tp, int pairs, const Lanes<float, K>& u,
-                                                 const Lanes<float, K>& t, Lanes<float, K>& q, Lanes<float, K>& q1,
-                                                 Lanes<float, K> (&S)[6]) {
-    for (int i = 0; i < pairs; ++i, tp += kChunks32 * W) {
-        const float4 a = tp[0], b = tp[W], c = tp[2 * W];
-        const float2 d = *(const float2*)(tp + 3 * W);
-        fieldRow<float, K>(a.x, a.z, a.w, b.x, b.y, b.z, b.w, u, t, q, q1, S);
-        fieldRow<float, K>(a.y, c.x, c.y, c.z, c.w, d.x, d.y, u, t, q, q1, S);
+static __device__ __forceinline__ void rowPair(const float4* __restrict__ tp, const Lanes<float, K>& u,
+                                               const Lanes<float, K>& t, Lanes<float, K>& q, Lanes<float, K>& q1,
+                                               Lanes<float, K> (&S)[6]) {
+    const float4 a = tp[0], b = tp[W], c = tp[2 * W];
+    const float2 d = *(const float2*)(tp + 3 * W);
+    fieldRow<float, K>(a.x, a.z, a.w, b.x, b.y, b.z, b.w, u, t, q, q1, S);
+    fieldRow<float, K>(a.y, c.x, c.y, c.z, c.w, d.x, d.y, u, t, q, q1, S);
+}
+// `pairs` row pairs of a column from its first 16-byte chunk.  LDS: a staged tile is
+// read by shared-memory loads, in a loop of its own, two row pairs an
+// iteration.  Such a load whose lanes differ in at most two addresses (W <=
+// 2) takes 2 cycles of an SM per 16 bytes of a warp, a generic load 4, and
+// the column loop of one lane per object was bound by the latter (82 % of the
+// load path's peak, FP64 pipe 52 %): 200,000 uneven objects x 8 steps FP64
+// 66.3 -> 60.5 ms, 10^6 x 4 split 110 -> 100; at four lanes the shorter
+// latency shows, 10^4 LEO x 20 FP64 14.9 -> 13.7.  The kernels of 168
+// registers keep one generic loop: with two they spill inside them (two
+// lanes, pairs, 10^4 LEO: 21.0 against 27.0 ms).
+template <typename T, int K, int W, bool LDS>
+static __device__ __forceinline__ void fieldRows(const TileRef& tile, int chunk, int pairs, const Lanes<T, K>& u,
+                                                 const Lanes<T, K>& t, Lanes<T, K>& q, Lanes<T, K>& q1,
+                                                 Lanes<T, K> (&S)[6]) {
+    using Chunk = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
+    constexpr int kStep = (sizeof(T) == 8 ? kChunks64 : kChunks32) * W;
+    if (LDS && tile.staged) {
+        const Chunk* tp = (const Chunk*)g_smem + chunk;
+#pragma unroll 2
+        for (int i = 0; i < pairs; ++i, tp += kStep) rowPair<K, W>(tp, u, t, q, q1, S);
+        return;
     }
+    const Chunk* __restrict__ tp = (const Chunk*)(!LDS && tile.staged ? (const void*)g_smem : tile.global) + chunk;
+    for (int i = 0; i < pairs; ++i, tp += kStep) rowPair<K, W>(tp, u, t, q, q1, S);
 }
 
 // Per-object quantities of the column sums.
@@ -322,8 +353,8 @@ static __device__ __forceinline__ void tidePart(const Rec& rec, int j, double x,
 // each at its best shape: 10^4 LEO objects x 20 steps at degree 70 FP64 20.1
 // -> 16.2, split 19.3 -> 13.9; 200,000 uneven objects x 8 steps FP64 121 ->
 // 86.6; 10^6 x 4 split 239 -> 126; 10^5 LEO x 4 at degree 120 split 62 -> 37.
-template <int L, int K, typename T, class Rec>
-static __device__ __forceinline__ void fieldAccel(const StepParams& p, const void* tile, const int4* __restrict__ blocks,
+template <int L, int K, typename T, bool LDS, class Rec>
+static __device__ __forceinline__ void fieldAccel(const StepParams& p, const TileRef& tile, const int4* __restrict__ blocks,
                                                   int nblocks, const Rec& rec, double x, double y, double z,
                                                   double out[3]) {
     constexpr int W = K * L;
@@ -371,7 +402,7 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const voi
         for (int k = 0; k < K; ++k) q.set(k, g[k].mag);
         const int low = kSplit ? p.lowDeg : N;
         const bool act = M < p.columns;
-        fieldRows<K, W>((const double2*)tile + blk.x + pj, act ? rowPairs64(M, N, low) : 0, u, t, q, q1, S);
+        fieldRows<double, K, W, LDS>(tile, blk.x + pj, act ? rowPairs64(M, N, low) : 0, u, t, q, q1, S);
         if constexpr (kSplit) {
             Lanes<T, K> qT = Lanes<T, K>::all(T(0)), qT1 = qT, ST[6];
 #pragma unroll
@@ -381,7 +412,7 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const voi
                 qT.set(k, q.get(k));
                 qT1.set(k, q1.get(k));
             }
-            fieldRows<K, W>((const float4*)tile + blk.z + pj, act ? rowPairs32(M, N, low) : 0, uT, tT, qT, qT1, ST);
+            fieldRows<T, K, W, LDS>(tile, blk.z + pj, act ? rowPairs32(M, N, low) : 0, uT, tT, qT, qT1, ST);
 #pragma unroll
             for (int c = 0; c < 6; ++c)
 #pragma unroll

@@ -421,8 +421,8 @@ static __device__ __noinline__ void tideAloneAccel(const Rec r, const double pos
 // full right-hand side acceleration (km/s^2); every lane of the group calls it.
 // PAIR: two lane groups share their columns (a separate kernel instantiation,
 // so the one-object-per-lane kernel keeps its own register allocation).
-template <int L, typename T, bool PAIR, class Rec>
-static __device__ __forceinline__ void accelerations(const StepParams& p, const void* tile,
+template <int L, typename T, bool PAIR, bool LDS, class Rec>
+static __device__ __forceinline__ void accelerations(const StepParams& p, const TileRef& tile,
                                               const Rec& r, const double pos[3], const double vel[3],
                                               double bc, double ams, double acc[3]) {
     const DevEnv& e = p.env;
@@ -474,9 +474,9 @@ static __device__ __forceinline__ void accelerations(const StepParams& p, const 
             // keep every row in FP64 (from the FP64 tile in global memory)
             if (!PAIR && sizeof(T) == 4 && p.splitRadius > 0.0
                 && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius)
-                fieldAccel<L, 1, double>(p, p.tile64, p.blocks64, p.nblocks64, r, bx, by, bz, a);
+                fieldAccel<L, 1, double, false>(p, TileRef{p.tile64, false}, p.blocks64, p.nblocks64, r, bx, by, bz, a);
             else
-                fieldAccel<L, PAIR ? 2 : 1, T>(p, tile, p.blocks, p.nblocks, r, bx, by, bz, a);
+                fieldAccel<L, PAIR ? 2 : 1, T, LDS>(p, tile, p.blocks, p.nblocks, r, bx, by, bz, a);
             double ai[3];
             if (isEarth) {
                 fromBody(r, a, ai);
@@ -701,8 +701,7 @@ static __device__ __forceinline__ RecordInterp recordFromGrid(const StepParams& 
 template <int L, typename T, bool SHARED_GRID, bool PAIR, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant__ StepParams p) {
     constexpr int NA = Axes<L>::N;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const void* tile = p.tile;
+    TileRef tile{p.tile, false};
     int kOffset = 0;
     if (!SHARED_GRID && !p.gridPairs) {  // per-object time needs the batch's record grid
         if (threadIdx.x == 0) atomicExch(p.errorFlag, 3);
@@ -710,13 +709,13 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
     }
     if (p.useSmemTile) {
         const bool test = p.tileWaitTest != 0;
-        if (stageTile(smem, p.tile, p.tileBytes, !test, test ? 4096L : (1L << 24)))
-            tile = smem;
+        if (stageTile(g_smem, p.tile, p.tileBytes, !test, test ? 4096L : (1L << 24)))
+            tile.staged = true;
         else if (threadIdx.x == 0 && p.tileFallbacks)
             atomicAdd(p.tileFallbacks, 1);  // this CTA reads the tile from global memory
         kOffset = p.tileBytes;
     }
-    const StageStore kst{(double*)(smem + kOffset) + threadIdx.x / L, (int)blockDim.x / L};
+    const StageStore kst{(double*)(g_smem + kOffset) + threadIdx.x / L, (int)blockDim.x / L};
     const int lane = (int)(threadIdx.x & 31);
     const int j = lane % L;
     const int g = lane / L;
@@ -800,11 +799,11 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
                 }
                 if (SHARED_GRID) {
                     const RecordRef rec{p.records + kstep * 13 + s};
-                    accelerations<L, T, PAIR>(p, tile, rec, st, st + 3, bc, ams, acc);
+                    accelerations<L, T, PAIR, MAXT <= kDeepThreads>(p, tile, rec, st, st + 3, bc, ams, acc);
                 } else {
                     const double ts = s == 0 ? t0 : t0 + dt * rkC(s - 1);
                     const RecordInterp rec = recordFromGrid(p, ts);
-                    accelerations<L, T, PAIR>(p, tile, rec, st, st + 3, bc, ams, acc);
+                    accelerations<L, T, PAIR, MAXT <= kDeepThreads>(p, tile, rec, st, st + 3, bc, ams, acc);
                 }
                 if (s < 12) {
 #pragma unroll
