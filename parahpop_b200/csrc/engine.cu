@@ -1073,7 +1073,6 @@ Engine::~Engine() {
     if (pairCache_) cudaFree(pairCache_);
     for (auto& kv : tiles_) {
         cudaFree(kv.second.dTile);
-        cudaFree(kv.second.dBlocks);
     }
 }
 
@@ -1101,7 +1100,6 @@ void Engine::uploadEnvironment() {
                            : n > h.shDegree || m > h.shOrder ? 0.0
                            : h.shNormalized ? 1.0 : 1.0 / normFactor(n, m);
     }
-    columns_ = h.hasShape ? fieldOrder(h) + 2 : 0;
     e.nbodies = (int)h.bodies.size();
     e.sunIndex = e.moonIndex = e.earthIndex = -1;
     int anyOcc = 0;
@@ -1283,11 +1281,10 @@ const Engine::Tile& Engine::tileFor(int L, bool split, int lowDeg) {
     const HostTile h = buildTile(host_, L, split, lowDeg);
     Tile tile;
     tile.nblocks = h.nblocks;
+    tile.chunk32 = h.chunk32;
     tile.bytes = (int)h.bytes.size();
     PHOP_CUDA(cudaMalloc(&tile.dTile, h.bytes.size()));
     PHOP_CUDA(cudaMemcpy(tile.dTile, h.bytes.data(), h.bytes.size(), cudaMemcpyHostToDevice));
-    PHOP_CUDA(cudaMalloc(&tile.dBlocks, h.blocks.size() * sizeof(int4)));
-    PHOP_CUDA(cudaMemcpy(tile.dBlocks, h.blocks.data(), h.blocks.size() * sizeof(int4), cudaMemcpyHostToDevice));
     return tiles_.emplace(key, tile).first->second;
 }
 
@@ -1501,18 +1498,15 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     const Tile& tile = tileFor(p.pairSh ? 2 * L : L, opt.split, lowDeg);
     p.tile = tile.dTile;
     p.tileBytes = tile.bytes;
-    p.blocks = tile.dBlocks;
     p.nblocks = tile.nblocks;
-    p.columns = columns_;
+    p.chunk32 = tile.chunk32;
     p.lowDeg = lowDeg;
     p.tile64 = nullptr;
-    p.blocks64 = nullptr;
     p.nblocks64 = 0;
     p.splitRadius = 0.0;
     if (opt.split && opt.splitFloorKm > 0.0) {
         const Tile& full = tileFor(L, false, lowDeg);
         p.tile64 = full.dTile;
-        p.blocks64 = full.dBlocks;
         p.nblocks64 = full.nblocks;
         p.splitRadius = host_.shR + opt.splitFloorKm;
     }

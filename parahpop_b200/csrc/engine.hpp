@@ -204,9 +204,8 @@ public:
     // internal
     struct Tile {
         void* dTile = nullptr;
-        int4* dBlocks = nullptr;
         int bytes = 0;
-        int nblocks = 0;
+        int nblocks = 0, chunk32 = 0;
     };
 
     // Launch geometry of one step-kernel launch.
@@ -275,7 +274,6 @@ private:
     std::map<std::string, std::pair<void*, size_t>> scratch_;
     std::map<int, Tile> tiles_;
     std::map<int, HostTile> hostTiles_;
-    int columns_ = 0;  // orders 0 .. columns_ - 1 of the geopotential tile have rows
     std::map<int, int> tuned_;  // autotuned lane count per batch class
     std::map<int64_t, int> occupancy_;  // resident CTAs per SM by launch configuration
     std::map<int, std::pair<int, int>> attrs_;  // maxThreadsPerBlock, numRegs of each step-kernel instantiation

@@ -46,7 +46,6 @@ struct Row {
 HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
     HostTile out;
     if (!h.hasShape) {
-        out.blocks.assign(1, int4{0, 0, 0, 0});
         out.bytes.assign(16, 0);
         return out;
     }
@@ -109,23 +108,17 @@ HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
     std::vector<double> f64;
     std::vector<float> f32;
     for (int b = 0; b < out.nblocks; ++b) {
-        int4 blk{(int)(f64.size() / 2), 0, (int)(f32.size() / 4), 0};
-        // lanes of a block run their own number of pairs; the first column has the most FP64 pairs
-        int p64 = 0, p32 = 0;
-        for (int j = 0; j < W && b * W + j < columns; ++j) {
-            p64 = std::max(p64, rowPairs64(b * W + j, N, low));
-            p32 = std::max(p32, rowPairs32(b * W + j, N, low));
-        }
+        const int n64 = rowPairs64(b * W, N, low), n32 = rowPairs32(b * W, N, low);
         const size_t base64 = f64.size(), base32 = f32.size();
-        f64.resize(base64 + (size_t)p64 * kChunks64 * W * 2, 0.0);
-        f32.resize(base32 + (size_t)p32 * kChunks32 * W * 4, 0.0f);
+        f64.resize(base64 + (size_t)n64 * kChunks64 * W * 2, 0.0);
+        f32.resize(base32 + (size_t)n32 * kChunks32 * W * 4, 0.0f);
         for (int j = 0; j < W; ++j) {
             const int M = b * W + j;
             if (M >= columns) break;
             const std::vector<Row> rows = column(M);
-            const int n64 = rowPairs64(M, N, low), n32 = rowPairs32(M, N, low);
             auto at = [&](int i) { return i < (int)rows.size() ? rows[i] : Row{}; };
-            for (int i = 0; i < n64; ++i) {
+            const int own64 = rowPairs64(M, N, low);
+            for (int i = 0; i < (split ? own64 : n64); ++i) {
                 const Row r0 = at(2 * i), r1 = at(2 * i + 1);
                 const double v[14] = {r0.a,    r1.a,    r0.x[0], r0.x[1], r0.x[2], r0.x[3], r0.x[4],
                                       r0.x[5], r1.x[0], r1.x[1], r1.x[2], r1.x[3], r1.x[4], r1.x[5]};
@@ -133,7 +126,7 @@ HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
                     std::memcpy(&f64[base64 + (((size_t)i * kChunks64 + c) * W + j) * 2], v + 2 * c, 16);
             }
             for (int i = 0; i < n32; ++i) {
-                const Row r0 = at(2 * n64 + 2 * i), r1 = at(2 * n64 + 2 * i + 1);
+                const Row r0 = at(2 * own64 + 2 * i), r1 = at(2 * own64 + 2 * i + 1);
                 const float v[16] = {(float)r0.a,    (float)r1.a,    (float)r0.x[0], (float)r0.x[1],
                                      (float)r0.x[2], (float)r0.x[3], (float)r0.x[4], (float)r0.x[5],
                                      (float)r1.x[0], (float)r1.x[1], (float)r1.x[2], (float)r1.x[3],
@@ -142,11 +135,8 @@ HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
                     std::memcpy(&f32[base32 + (((size_t)i * kChunks32 + c) * W + j) * 4], v + 4 * c, 16);
             }
         }
-        out.blocks.push_back(blk);
     }
-    // FP32 rows follow the FP64 rows
-    const int base32 = (int)(f64.size() / 2);
-    for (int4& blk : out.blocks) blk.z += base32;
+    out.chunk32 = (int)(f64.size() / 2);
     out.bytes.resize(f64.size() * 8 + f32.size() * 4 + 16, 0);
     std::memcpy(out.bytes.data(), f64.data(), f64.size() * 8);
     std::memcpy(out.bytes.data() + f64.size() * 8, f32.data(), f32.size() * 4);

@@ -121,31 +121,47 @@ static __device__ __forceinline__ void fieldRow(T a, T xc, T xs, T yc, T ys, T z
 extern __shared__ __align__(128) unsigned char g_smem[];
 struct TileRef {
     const void* global;
+    int nblocks, chunk32;
     bool staged;
 };
 
-// One row pair of a column, W lanes interleaved.
-template <int K, int W>
-static __device__ __forceinline__ void rowPair(const double2* __restrict__ tp, const Lanes<double, K>& u,
-                                               const Lanes<double, K>& t, Lanes<double, K>& q, Lanes<double, K>& q1,
-                                               Lanes<double, K> (&S)[6]) {
-    const double2 a = tp[0], x0 = tp[W], y0 = tp[2 * W], z0 = tp[3 * W];
-    const double2 x1 = tp[4 * W], y1 = tp[5 * W], z1 = tp[6 * W];
-    fieldRow<double, K>(a.x, x0.x, x0.y, y0.x, y0.y, z0.x, z0.y, u, t, q, q1, S);
-    fieldRow<double, K>(a.y, x1.x, x1.y, y1.x, y1.y, z1.x, z1.y, u, t, q, q1, S);
-}
-template <int K, int W>
-static __device__ __forceinline__ void rowPair(const float4* __restrict__ tp, const Lanes<float, K>& u,
-                                               const Lanes<float, K>& t, Lanes<float, K>& q, Lanes<float, K>& q1,
-                                               Lanes<float, K> (&S)[6]) {
-    const float4 a = tp[0], b = tp[W], c = tp[2 * W];
-    const float2 d = *(const float2*)(tp + 3 * W);
-    fieldRow<float, K>(a.x, a.z, a.w, b.x, b.y, b.z, b.w, u, t, q, q1, S);
-    fieldRow<float, K>(a.y, c.x, c.y, c.z, c.w, d.x, d.y, u, t, q, q1, S);
-}
+// The chunks of one row pair of a lane, W lanes interleaved.
+template <typename T> struct PairRows;
+template <> struct PairRows<double> {
+    static constexpr int kChunks = kChunks64;
+    double2 c[kChunks64];
+    template <int W> __device__ __forceinline__ void load(const double2* __restrict__ tp) {
+#pragma unroll
+        for (int i = 0; i < kChunks64; ++i) c[i] = tp[i * W];
+    }
+    template <int K>
+    __device__ __forceinline__ void add(const Lanes<double, K>& u, const Lanes<double, K>& t, Lanes<double, K>& q,
+                                        Lanes<double, K>& q1, Lanes<double, K> (&S)[6]) const {
+        fieldRow<double, K>(c[0].x, c[1].x, c[1].y, c[2].x, c[2].y, c[3].x, c[3].y, u, t, q, q1, S);
+        fieldRow<double, K>(c[0].y, c[4].x, c[4].y, c[5].x, c[5].y, c[6].x, c[6].y, u, t, q, q1, S);
+    }
+};
+template <> struct PairRows<float> {
+    static constexpr int kChunks = kChunks32;
+    float4 a, b, c;
+    float2 d;
+    template <int W> __device__ __forceinline__ void load(const float4* __restrict__ tp) {
+        a = tp[0];
+        b = tp[W];
+        c = tp[2 * W];
+        d = *(const float2*)(tp + 3 * W);
+    }
+    template <int K>
+    __device__ __forceinline__ void add(const Lanes<float, K>& u, const Lanes<float, K>& t, Lanes<float, K>& q,
+                                        Lanes<float, K>& q1, Lanes<float, K> (&S)[6]) const {
+        fieldRow<float, K>(a.x, a.z, a.w, b.x, b.y, b.z, b.w, u, t, q, q1, S);
+        fieldRow<float, K>(a.y, c.x, c.y, c.z, c.w, d.x, d.y, u, t, q, q1, S);
+    }
+};
 // `pairs` row pairs of a column from its first 16-byte chunk.  LDS: a staged tile is
 // read by shared-memory loads, in a loop of its own, two row pairs an
-// iteration.  Such a load whose lanes differ in at most two addresses (W <=
+// iteration (four in FP32: one CTA of eight warps, one lane per object, 82.7
+// against 85.7 thousand cycles an evaluation at degree 70).  Such a load whose lanes differ in at most two addresses (W <=
 // 2) takes 2 cycles of an SM per 16 bytes of a warp, a generic load 4, and
 // the column loop of one lane per object was bound by the latter (82 % of the
 // load path's peak, FP64 pipe 52 %): 200,000 uneven objects x 8 steps FP64
@@ -158,15 +174,23 @@ static __device__ __forceinline__ void fieldRows(const TileRef& tile, int chunk,
                                                  const Lanes<T, K>& t, Lanes<T, K>& q, Lanes<T, K>& q1,
                                                  Lanes<T, K> (&S)[6]) {
     using Chunk = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
-    constexpr int kStep = (sizeof(T) == 8 ? kChunks64 : kChunks32) * W;
+    constexpr int kStep = PairRows<T>::kChunks * W;
     if (LDS && tile.staged) {
         const Chunk* tp = (const Chunk*)g_smem + chunk;
-#pragma unroll 2
-        for (int i = 0; i < pairs; ++i, tp += kStep) rowPair<K, W>(tp, u, t, q, q1, S);
+#pragma unroll(sizeof(T) == 8 ? 2 : 4)
+        for (int i = 0; i < pairs; ++i, tp += kStep) {
+            PairRows<T> r;
+            r.template load<W>(tp);
+            r.template add<K>(u, t, q, q1, S);
+        }
         return;
     }
     const Chunk* __restrict__ tp = (const Chunk*)(!LDS && tile.staged ? (const void*)g_smem : tile.global) + chunk;
-    for (int i = 0; i < pairs; ++i, tp += kStep) rowPair<K, W>(tp, u, t, q, q1, S);
+    for (int i = 0; i < pairs; ++i, tp += kStep) {
+        PairRows<T> r;
+        r.template load<W>(tp);
+        r.template add<K>(u, t, q, q1, S);
+    }
 }
 
 // Per-object quantities of the column sums.
@@ -354,8 +378,7 @@ static __device__ __forceinline__ void tidePart(const Rec& rec, int j, double x,
 // -> 16.2, split 19.3 -> 13.9; 200,000 uneven objects x 8 steps FP64 121 ->
 // 86.6; 10^6 x 4 split 239 -> 126; 10^5 LEO x 4 at degree 120 split 62 -> 37.
 template <int L, int K, typename T, bool LDS, class Rec>
-static __device__ __forceinline__ void fieldAccel(const StepParams& p, const TileRef& tile, const int4* __restrict__ blocks,
-                                                  int nblocks, const Rec& rec, double x, double y, double z,
+static __device__ __forceinline__ void fieldAccel(const StepParams& p, const TileRef& tile, const Rec& rec, double x, double y, double z,
                                                   double out[3]) {
     constexpr int W = K * L;
     constexpr bool kSplit = sizeof(T) == 4;
@@ -392,17 +415,25 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const Til
             tT.set(k, g[k].t);
         }
     }
-    for (int b = 0; b < nblocks; ++b) {
-        const int M = b * W + pj;
-        const int4 blk = blocks[b];
+    const int low = kSplit ? p.lowDeg : N;
+    int at64 = pj, at32 = tile.chunk32 + pj;  // the lane's first chunks of the block
+    for (int b = 0; b < tile.nblocks; ++b) {
+        const int n64 = rowPairs64(b * W, N, low);
         Lanes<double, K> q, q1 = Lanes<double, K>::all(0.0), S[6];
 #pragma unroll
         for (int c = 0; c < 6; ++c) S[c] = Lanes<double, K>::all(0.0);
+        double cL[K], sL[K];
 #pragma unroll
-        for (int k = 0; k < K; ++k) q.set(k, g[k].mag);
-        const int low = kSplit ? p.lowDeg : N;
-        const bool act = M < p.columns;
-        fieldRows<double, K, W, LDS>(tile, blk.x + pj, act ? rowPairs64(M, N, low) : 0, u, t, q, q1, S);
+        for (int k = 0; k < K; ++k) {
+            q.set(k, g[k].mag);
+            cL[k] = g[k].cL;
+            sL[k] = g[k].sL;
+            g[k].cL = __fma_rn(g[k].cW, cL[k], -__dmul_rn(g[k].sW, sL[k]));
+            g[k].sL = __fma_rn(g[k].cW, sL[k], __dmul_rn(g[k].sW, cL[k]));
+            g[k].mag = __dmul_rn(g[k].mag, g[k].magW);
+        }
+        fieldRows<double, K, W, LDS>(tile, at64, kSplit ? rowPairs64(b * W + pj, N, low) : n64, u, t, q, q1, S);
+        at64 += n64 * kChunks64 * W;
         if constexpr (kSplit) {
             Lanes<T, K> qT = Lanes<T, K>::all(T(0)), qT1 = qT, ST[6];
 #pragma unroll
@@ -412,22 +443,19 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const Til
                 qT.set(k, q.get(k));
                 qT1.set(k, q1.get(k));
             }
-            fieldRows<T, K, W, LDS>(tile, blk.z + pj, act ? rowPairs32(M, N, low) : 0, uT, tT, qT, qT1, ST);
+            const int n32 = rowPairs32(b * W, N, low);
+            fieldRows<T, K, W, LDS>(tile, at32, n32, uT, tT, qT, qT1, ST);
+            at32 += n32 * kChunks32 * W;
 #pragma unroll
             for (int c = 0; c < 6; ++c)
 #pragma unroll
                 for (int k = 0; k < K; ++k) S[c].v[k] = __dadd_rn(S[c].v[k], ST[c].get(k));
         }
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
+        for (int k = 0; k < K; ++k)
 #pragma unroll
             for (int c = 0; c < 3; ++c)
-                g[k].acc[c] = __fma_rn(g[k].cL, S[2 * c].v[k], __fma_rn(g[k].sL, S[2 * c + 1].v[k], g[k].acc[c]));
-            const double c = __fma_rn(g[k].cW, g[k].cL, -__dmul_rn(g[k].sW, g[k].sL));
-            g[k].sL = __fma_rn(g[k].cW, g[k].sL, __dmul_rn(g[k].sW, g[k].cL));
-            g[k].cL = c;
-            g[k].mag = __dmul_rn(g[k].mag, g[k].magW);
-        }
+                g[k].acc[c] = __fma_rn(cL[k], S[2 * c].v[k], __fma_rn(sL[k], S[2 * c + 1].v[k], g[k].acc[c]));
     }
     // fold the set's partial sums of each object
 #pragma unroll

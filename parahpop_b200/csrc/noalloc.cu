@@ -10,7 +10,7 @@
 // one file-scope device array, kStaticScratchBytes large, carved as:
 //
 //   control words (work counter, error flag)     256 B
-//   coefficient tile + block table               kTileBytes + kBlockBytes
+//   coefficient tile                             kTileBytes
 //   step start / size tables                     2 x kMaxSteps doubles
 //   stage epochs                                 13 x kMaxSteps doubles
 //   epoch records                                13 x kMaxSteps records
@@ -44,7 +44,6 @@ constexpr size_t kStaticScratchBytes = 4u << 20;
 constexpr int kMaxSteps = 256;
 constexpr size_t kCtlBytes = 256;
 constexpr size_t kTileBytes = 640u << 10;
-constexpr size_t kBlockBytes = 4u << 10;
 
 static __device__ __align__(256) unsigned char g_staticScratch[kStaticScratchBytes];
 
@@ -57,7 +56,7 @@ struct DeviceScratch {
 DeviceScratch g_scratch[64];
 std::mutex g_scratchMutex;
 
-static_assert(kCtlBytes + kTileBytes + kBlockBytes + 2 * kMaxSteps * sizeof(double) + 13 * kMaxSteps * sizeof(double)
+static_assert(kCtlBytes + kTileBytes + 2 * kMaxSteps * sizeof(double) + 13 * kMaxSteps * sizeof(double)
                       + 13 * kMaxSteps * sizeof(EpochRecord) + 1024
                   <= kStaticScratchBytes,
               "static scratch layout does not fit");
@@ -144,8 +143,6 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     p += kCtlBytes;
     void* tileDst = p;
     p += kTileBytes;
-    int4* blocksDst = (int4*)p;
-    p += kBlockBytes;
     double* dT0 = (double*)p;
     p += kMaxSteps * sizeof(double);
     double* dDt = (double*)p;
@@ -159,7 +156,7 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     if (host_.hasShape && !withinTileLimit(host_.shDegree, host_.shOrder, L, opt.split, lowDeg))
         throw std::runtime_error("coefficient tile exceeds the allocation-free entry point's 512 KiB limit");
     const HostTile& ht = hostTileFor(L, opt.split, lowDeg);
-    if (ht.bytes.size() > kTileBytes || ht.blocks.size() * sizeof(int4) > kBlockBytes)
+    if (ht.bytes.size() > kTileBytes)
         throw std::runtime_error("coefficient tile exceeds the allocation-free entry point's 512 KiB limit");
     const int key = (lowDeg * 32 + L) * 2 + (opt.split ? 1 : 0);
     auto check = [](cudaError_t e) {
@@ -173,8 +170,6 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
         if (ds.tileOwner != serial_ || ds.tileKey != key) {
             ds.tileOwner = 0;
             check(cudaMemcpyAsync(tileDst, ht.bytes.data(), ht.bytes.size(), cudaMemcpyHostToDevice, stream));
-            check(cudaMemcpyAsync(blocksDst, ht.blocks.data(), ht.blocks.size() * sizeof(int4),
-                                  cudaMemcpyHostToDevice, stream));
             ds.tileOwner = serial_;
             ds.tileKey = key;
         }
@@ -198,9 +193,8 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.maxSteps = maxSteps;
     sp.tile = tileDst;
     sp.tileBytes = (int)ht.bytes.size();
-    sp.blocks = blocksDst;
     sp.nblocks = ht.nblocks;
-    sp.columns = columns_;
+    sp.chunk32 = ht.chunk32;
     sp.lowDeg = lowDeg;
     sp.workCounter = ctl;
     sp.errorFlag = ctl + 1;

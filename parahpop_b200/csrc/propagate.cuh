@@ -86,12 +86,10 @@ struct StepParams {
     // geopotential
     const void* tile;       // tile entries in global memory
     int tileBytes;          // multiple of 16
-    const int4* blocks;     // per block of columns: first FP64 and FP32 chunk (geopotential.hpp)
-    int nblocks;
-    int columns;            // orders 0 .. columns - 1 have rows
-    int lowDeg;             // split precision: rows of degrees n <= lowDeg are FP64
-    const void* tile64;     // split precision: the FP64 tile (global memory) of L lanes, its blocks
-    const int4* blocks64;
+    int nblocks;            // blocks of columns
+    int chunk32;            // split precision: 16-byte chunks of FP64 rows before the FP32 rows
+    int lowDeg;             // split precision: FP64 low part
+    const void* tile64;     // split precision: the FP64 tile (global memory) of L lanes
     int nblocks64;
     double splitRadius;     // split precision: radius (km) below which the tile part stays FP64; 0 = none
     int useSmemTile;

@@ -474,9 +474,9 @@ static __device__ __forceinline__ void accelerations(const StepParams& p, const 
             // keep every row in FP64 (from the FP64 tile in global memory)
             if (!PAIR && sizeof(T) == 4 && p.splitRadius > 0.0
                 && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius)
-                fieldAccel<L, 1, double, false>(p, TileRef{p.tile64, false}, p.blocks64, p.nblocks64, r, bx, by, bz, a);
+                fieldAccel<L, 1, double, false>(p, TileRef{p.tile64, p.nblocks64, 0, false}, r, bx, by, bz, a);
             else
-                fieldAccel<L, PAIR ? 2 : 1, T, LDS>(p, tile, p.blocks, p.nblocks, r, bx, by, bz, a);
+                fieldAccel<L, PAIR ? 2 : 1, T, LDS>(p, tile, r, bx, by, bz, a);
             double ai[3];
             if (isEarth) {
                 fromBody(r, a, ai);
@@ -701,7 +701,7 @@ static __device__ __forceinline__ RecordInterp recordFromGrid(const StepParams& 
 template <int L, typename T, bool SHARED_GRID, bool PAIR, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant__ StepParams p) {
     constexpr int NA = Axes<L>::N;
-    TileRef tile{p.tile, false};
+    TileRef tile{p.tile, p.nblocks, p.chunk32, false};
     int kOffset = 0;
     if (!SHARED_GRID && !p.gridPairs) {  // per-object time needs the batch's record grid
         if (threadIdx.x == 0) atomicExch(p.errorFlag, 3);
