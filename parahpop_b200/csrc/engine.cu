@@ -1281,7 +1281,6 @@ const Engine::Tile& Engine::tileFor(int L, bool split, int lowDeg) {
     const HostTile h = buildTile(host_, L, split, lowDeg);
     Tile tile;
     tile.nblocks = h.nblocks;
-    tile.chunk32 = h.chunk32;
     tile.bytes = (int)h.bytes.size();
     PHOP_CUDA(cudaMalloc(&tile.dTile, h.bytes.size()));
     PHOP_CUDA(cudaMemcpy(tile.dTile, h.bytes.data(), h.bytes.size(), cudaMemcpyHostToDevice));
@@ -1499,7 +1498,6 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     p.tile = tile.dTile;
     p.tileBytes = tile.bytes;
     p.nblocks = tile.nblocks;
-    p.chunk32 = tile.chunk32;
     p.lowDeg = lowDeg;
     p.tile64 = nullptr;
     p.nblocks64 = 0;
@@ -1512,39 +1510,46 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     }
     // shared memory per CTA: the coefficient tile (when it fits) plus the
     // stage accelerations of its objects
+    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - bytes) / kStageBytes * L / 32 * 32; };
+    const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs));
+    const int staged = opt.tileSmem != 0 && tile.bytes + 1024 <= maxSmem_ ? fit(tile.bytes) : 0;
+    p.useSmemTile = staged >= 64;
+    // A tile that does not fit, or leaves room for fewer than three quarters
+    // of the threads, is streamed through a ring per warp where the kernel
+    // can (a streamed row costs about a fifth more than a staged one);
+    // "tile_smem" = 0 asks for reads through L1, and the FP64 floor of the
+    // split form lets a warp's objects part in the row loop.
+    const int streamed = (maxSmem_ - 1024) / (kRingBytes + kStageBytes * (32 / L)) * 32;
+    p.streamTile = opt.tileSmem != 0 && hasStream(L, p.deepRegs) && tile.nblocks > 0 && p.splitRadius == 0.0
+                   && std::min(staged, bound) < std::min(streamed, bound) * 3 / 4;
+    if (p.streamTile) p.useSmemTile = 0;
     int registers = 0;
-    int threadsReq = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs));
+    int threadsReq = bound;
     {
         // never more threads than the compiled instantiation accepts (its
         // register count times the threads must fit the SM's register file)
-        const int akey = (((L * 2 + (opt.split ? 1 : 0)) * 2 + (shared ? 1 : 0)) * 2 + p.pairSh) * 2 + p.deepRegs;
+        const int akey = ((((L * 2 + (opt.split ? 1 : 0)) * 2 + (shared ? 1 : 0)) * 2 + p.pairSh) * 2 + p.deepRegs) * 2
+                         + p.streamTile;
         auto at = attrs_.find(akey);
         if (at == attrs_.end()) {
             cudaFuncAttributes a{};
-            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, &a));
+            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, &a));
             at = attrs_.emplace(akey, std::make_pair(a.maxThreadsPerBlock, a.numRegs)).first;
         }
         threadsReq = std::max(32, std::min(threadsReq, at->second.first / 32 * 32));
         registers = at->second.second;
     }
-    int threads = threadsReq;
-    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - bytes) / kStageBytes * L / 32 * 32; };
-    if (opt.tileSmem != 0 && tile.bytes + 1024 <= maxSmem_ && fit(tile.bytes) >= 64) {
-        p.useSmemTile = 1;
-        threads = std::min(threadsReq, fit(tile.bytes));
-    } else {
-        p.useSmemTile = 0;
-        threads = std::min(threadsReq, fit(0));
-    }
+    int threads = std::min(threadsReq, p.useSmemTile ? staged : p.streamTile ? streamed : fit(0));
     int perSm = opt.ctasPerSm;
     if (perSm <= 0) {
         const int smem = propagateSmemBytes(p, L, threads);
         const int64_t key = (((((int64_t)smem * 1024 + threads) * 32 + L) * 4 + (opt.split ? 2 : 0) + (shared ? 1 : 0)) * 2
-                             + p.pairSh) * 2 + p.deepRegs;
+                             + p.pairSh) * 4 + p.deepRegs * 2 + p.streamTile;
         auto it = occupancy_.find(key);
         if (it == occupancy_.end())
             it = occupancy_
-                     .emplace(key, propagateMaxCtasPerSm(L, opt.split, shared, p.pairSh, p.deepRegs, threads, smem))
+                     .emplace(key, propagateMaxCtasPerSm(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, threads,
+                                                    smem))
                      .first;
         perSm = it->second;
     }

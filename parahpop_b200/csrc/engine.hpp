@@ -205,7 +205,7 @@ public:
     struct Tile {
         void* dTile = nullptr;
         int bytes = 0;
-        int nblocks = 0, chunk32 = 0;
+        int nblocks = 0;
     };
 
     // Launch geometry of one step-kernel launch.

@@ -46,7 +46,7 @@ struct Row {
 HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
     HostTile out;
     if (!h.hasShape) {
-        out.bytes.assign(16, 0);
+        out.bytes.assign(kStageChunks * 16, 0);
         return out;
     }
     const int N = h.shDegree, order = fieldOrder(h);
@@ -105,13 +105,12 @@ HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
     };
     const int columns = std::min(order, N) + 2;  // orders 0 .. order + 1
     out.nblocks = (columns + W - 1) / W;
-    std::vector<double> f64;
-    std::vector<float> f32;
     for (int b = 0; b < out.nblocks; ++b) {
         const int n64 = rowPairs64(b * W, N, low), n32 = rowPairs32(b * W, N, low);
-        const size_t base64 = f64.size(), base32 = f32.size();
-        f64.resize(base64 + (size_t)n64 * kChunks64 * W * 2, 0.0);
-        f32.resize(base32 + (size_t)n32 * kChunks32 * W * 4, 0.0f);
+        const size_t base = out.bytes.size();
+        out.bytes.resize(base + ((size_t)n64 * kChunks64 + (size_t)n32 * kChunks32) * W * 16, 0);
+        unsigned char* p64 = out.bytes.data() + base;
+        unsigned char* p32 = p64 + (size_t)n64 * kChunks64 * W * 16;
         for (int j = 0; j < W; ++j) {
             const int M = b * W + j;
             if (M >= columns) break;
@@ -123,7 +122,7 @@ HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
                 const double v[14] = {r0.a,    r1.a,    r0.x[0], r0.x[1], r0.x[2], r0.x[3], r0.x[4],
                                       r0.x[5], r1.x[0], r1.x[1], r1.x[2], r1.x[3], r1.x[4], r1.x[5]};
                 for (int c = 0; c < kChunks64; ++c)
-                    std::memcpy(&f64[base64 + (((size_t)i * kChunks64 + c) * W + j) * 2], v + 2 * c, 16);
+                    std::memcpy(p64 + (((size_t)i * kChunks64 + c) * W + j) * 16, v + 2 * c, 16);
             }
             for (int i = 0; i < n32; ++i) {
                 const Row r0 = at(2 * own64 + 2 * i), r1 = at(2 * own64 + 2 * i + 1);
@@ -132,14 +131,12 @@ HostTile buildTile(const HostEnvironment& h, int W, bool split, int lowDeg) {
                                      (float)r1.x[0], (float)r1.x[1], (float)r1.x[2], (float)r1.x[3],
                                      (float)r1.x[4], (float)r1.x[5], 0.f,            0.f};
                 for (int c = 0; c < kChunks32; ++c)
-                    std::memcpy(&f32[base32 + (((size_t)i * kChunks32 + c) * W + j) * 4], v + 4 * c, 16);
+                    std::memcpy(p32 + (((size_t)i * kChunks32 + c) * W + j) * 16, v + 4 * c, 16);
             }
         }
     }
-    out.chunk32 = (int)(f64.size() / 2);
-    out.bytes.resize(f64.size() * 8 + f32.size() * 4 + 16, 0);
-    std::memcpy(out.bytes.data(), f64.data(), f64.size() * 8);
-    std::memcpy(out.bytes.data() + f64.size() * 8, f32.data(), f32.size() * 4);
+    const size_t stage = kStageChunks * 16;
+    out.bytes.resize((out.bytes.size() + stage - 1) / stage * stage, 0);
     return out;
 }
 

@@ -116,13 +116,83 @@ static __device__ __forceinline__ void fieldRow(T a, T xc, T xs, T yc, T ys, T z
     q = n;
 }
 
-// The tile, in global memory or staged at the start of the CTA's dynamic
-// shared memory.
+// The tile: staged at the start of the CTA's dynamic shared memory, streamed
+// through the warp's ring (kernels that read shared memory by their own
+// loads), or read from global memory.
 extern __shared__ __align__(128) unsigned char g_smem[];
 struct TileRef {
     const void* global;
-    int nblocks, chunk32;
+    int nblocks;
     bool staged;
+};
+
+// The stream of a tile too large for shared memory: the warp copies it, stage
+// by stage (2 KiB, four 16-byte cp.async a lane), into a ring of eight stages
+// in shared memory, always five to six stages ahead of its row loop, and
+// starts over at the tile's end for the next evaluation.  A row (W chunks)
+// may be read once `ready` has passed it.  Stage k is acquired while the
+// reading row is in stage k - 1 at the earliest, so the slot of stage k - 2
+// is free then and takes the next copy.  The ring's first rows are repeated
+// past its end, so that a row pair is read at fixed offsets from its first
+// row.  Every lane of the warp makes every call.  The loads of a warp then
+// come from shared memory with hundreds of cycles of lead, instead of missing
+// L1 one row pair at a time: 10^5 LEO objects x 4 steps at degree 120 in
+// split precision 37.9 -> 26.7 ms, 20,011 in FP64 13.6 -> 11.1 (four
+// lanes; one lane 20.4 -> 13.1).
+template <int W>
+struct TileStream {
+    static constexpr unsigned kRows = kStageChunks / W;  // rows of a stage
+    static constexpr unsigned kMask = kRingStages * kRows - 1;
+    int base = 0;  // byte offset of the ring in g_smem
+    const uint4* src = nullptr;
+    int stages = 0, next = 0;
+    unsigned issued = 0, pos = 0, ready = 0;
+
+    __device__ __forceinline__ void issue() {
+        static_assert(W > 8 || 2 * kChunks64 <= kRows, "a stage holds two row pairs");
+        const int lane = (int)(threadIdx.x & 31), slot = (int)(issued & (kRingStages - 1));
+        const uint4* from = src + (size_t)next * kStageChunks + lane;
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(g_smem) + base + (slot * kStageChunks + lane) * 16;
+#pragma unroll
+        for (int i = 0; i < kStageChunks / 32; ++i)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + i * 512), "l"(from + i * 32) : "memory");
+        if (slot == 0) {
+#pragma unroll
+            for (int i = 0; i < (kRingMirror * W + 31) / 32; ++i)
+                if (lane + i * 32 < kRingMirror * W)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + kRingStages * kStageChunks * 16
+                                                                                   + i * 512),
+                                 "l"(from + i * 32)
+                                 : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        next = next + 1 == stages ? 0 : next + 1;
+        ++issued;
+    }
+    __device__ __forceinline__ void begin(int smemOffset, const void* tile, int bytes) {
+        base = smemOffset;
+        src = (const uint4*)tile;
+        stages = bytes / (kStageChunks * 16);
+        for (int k = 0; k < kRingStages - 2; ++k) issue();
+    }
+    // rows pos .. pos + rows - 1 readable (rows <= kRows)
+    __device__ __forceinline__ void need(unsigned rows) {
+        if ((int)(pos + rows - ready) > 0) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(kRingStages - 3) : "memory");
+            __syncwarp();
+            issue();
+            ready += kRows;
+        }
+    }
+    // the lane's chunk of the row `ahead` rows on
+    template <typename Chunk> __device__ __forceinline__ const Chunk* row(unsigned ahead, int pj) const {
+        return (const Chunk*)(g_smem + base) + ((pos + ahead) & kMask) * W + pj;
+    }
+    // the tile's padding at the end of an evaluation
+    __device__ __forceinline__ void rewind() { pos = ready; }
+    __device__ __forceinline__ void end() {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
 };
 
 // The chunks of one row pair of a lane, W lanes interleaved.
@@ -158,7 +228,7 @@ template <> struct PairRows<float> {
         fieldRow<float, K>(a.y, c.x, c.y, c.z, c.w, d.x, d.y, u, t, q, q1, S);
     }
 };
-// `pairs` row pairs of a column from its first 16-byte chunk.  LDS: a staged tile is
+// `pairs` row pairs of a column from its first 16-byte chunk.  kShared: a staged tile is
 // read by shared-memory loads, in a loop of its own, two row pairs an
 // iteration (four in FP32: one CTA of eight warps, one lane per object, 82.7
 // against 85.7 thousand cycles an evaluation at degree 70).  Such a load whose lanes differ in at most two addresses (W <=
@@ -169,14 +239,17 @@ template <> struct PairRows<float> {
 // latency shows, 10^4 LEO x 20 FP64 14.9 -> 13.7.  The kernels of 168
 // registers keep one generic loop: with two they spill inside them (two
 // lanes, pairs, 10^4 LEO: 21.0 against 27.0 ms).
-template <typename T, int K, int W, bool LDS>
-static __device__ __forceinline__ void fieldRows(const TileRef& tile, int chunk, int pairs, const Lanes<T, K>& u,
-                                                 const Lanes<T, K>& t, Lanes<T, K>& q, Lanes<T, K>& q1,
-                                                 Lanes<T, K> (&S)[6]) {
+// `room`: the pairs the block holds per lane (the stream passes them all);
+// ALL: pairs == room.
+enum class TileRead { kGeneric, kShared, kStream };  // see fieldRows; the kernel's instantiation
+template <typename T, int K, int W, TileRead MODE, bool ALL>
+static __device__ __forceinline__ void fieldRows(const TileRef& tile, TileStream<W>& stream, int pj, int chunk, int pairs,
+                                                 int room, const Lanes<T, K>& u, const Lanes<T, K>& t, Lanes<T, K>& q,
+                                                 Lanes<T, K>& q1, Lanes<T, K> (&S)[6]) {
     using Chunk = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
-    constexpr int kStep = PairRows<T>::kChunks * W;
-    if (LDS && tile.staged) {
-        const Chunk* tp = (const Chunk*)g_smem + chunk;
+    constexpr int kChunks = PairRows<T>::kChunks, kStep = kChunks * W;
+    if (MODE == TileRead::kShared && tile.staged) {
+        const Chunk* tp = (const Chunk*)g_smem + chunk + pj;
 #pragma unroll(sizeof(T) == 8 ? 2 : 4)
         for (int i = 0; i < pairs; ++i, tp += kStep) {
             PairRows<T> r;
@@ -185,7 +258,28 @@ static __device__ __forceinline__ void fieldRows(const TileRef& tile, int chunk,
         }
         return;
     }
-    const Chunk* __restrict__ tp = (const Chunk*)(!LDS && tile.staged ? (const void*)g_smem : tile.global) + chunk;
+    if constexpr (MODE == TileRead::kStream) {
+        int i = 0;
+        for (; i + 1 < room; i += 2) {
+            stream.need(2 * kChunks);
+            PairRows<T> r0, r1;
+            r0.template load<W>(stream.template row<Chunk>(0, pj));
+            r1.template load<W>(stream.template row<Chunk>(kChunks, pj));
+            stream.pos += 2 * kChunks;
+            if (ALL || i < pairs) r0.template add<K>(u, t, q, q1, S);
+            if (ALL || i + 1 < pairs) r1.template add<K>(u, t, q, q1, S);
+        }
+        if (i < room) {
+            stream.need(kChunks);
+            PairRows<T> r;
+            r.template load<W>(stream.template row<Chunk>(0, pj));
+            stream.pos += kChunks;
+            if (ALL || i < pairs) r.template add<K>(u, t, q, q1, S);
+        }
+        return;
+    }
+    const Chunk* __restrict__ tp =
+        (const Chunk*)(MODE == TileRead::kGeneric && tile.staged ? (const void*)g_smem : tile.global) + chunk + pj;
     for (int i = 0; i < pairs; ++i, tp += kStep) {
         PairRows<T> r;
         r.template load<W>(tp);
@@ -377,9 +471,9 @@ static __device__ __forceinline__ void tidePart(const Rec& rec, int j, double x,
 // each at its best shape: 10^4 LEO objects x 20 steps at degree 70 FP64 20.1
 // -> 16.2, split 19.3 -> 13.9; 200,000 uneven objects x 8 steps FP64 121 ->
 // 86.6; 10^6 x 4 split 239 -> 126; 10^5 LEO x 4 at degree 120 split 62 -> 37.
-template <int L, int K, typename T, bool LDS, class Rec>
-static __device__ __forceinline__ void fieldAccel(const StepParams& p, const TileRef& tile, const Rec& rec, double x, double y, double z,
-                                                  double out[3]) {
+template <int L, int K, typename T, TileRead MODE, class Rec>
+static __device__ __forceinline__ void fieldAccel(const StepParams& p, const TileRef& tile, TileStream<K * L>& stream,
+                                                  const Rec& rec, double x, double y, double z, double out[3]) {
     constexpr int W = K * L;
     constexpr bool kSplit = sizeof(T) == 4;
     const int lane = (int)(threadIdx.x & 31);
@@ -416,7 +510,7 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const Til
         }
     }
     const int low = kSplit ? p.lowDeg : N;
-    int at64 = pj, at32 = tile.chunk32 + pj;  // the lane's first chunks of the block
+    int at = 0;  // the block's first chunk
     for (int b = 0; b < tile.nblocks; ++b) {
         const int n64 = rowPairs64(b * W, N, low);
         Lanes<double, K> q, q1 = Lanes<double, K>::all(0.0), S[6];
@@ -432,8 +526,9 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const Til
             g[k].sL = __fma_rn(g[k].cW, sL[k], __dmul_rn(g[k].sW, cL[k]));
             g[k].mag = __dmul_rn(g[k].mag, g[k].magW);
         }
-        fieldRows<double, K, W, LDS>(tile, at64, kSplit ? rowPairs64(b * W + pj, N, low) : n64, u, t, q, q1, S);
-        at64 += n64 * kChunks64 * W;
+        fieldRows<double, K, W, MODE, !kSplit>(tile, stream, pj, at, kSplit ? rowPairs64(b * W + pj, N, low) : n64, n64, u,
+                                              t, q, q1, S);
+        at += n64 * kChunks64 * W;
         if constexpr (kSplit) {
             Lanes<T, K> qT = Lanes<T, K>::all(T(0)), qT1 = qT, ST[6];
 #pragma unroll
@@ -444,8 +539,8 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const Til
                 qT1.set(k, q1.get(k));
             }
             const int n32 = rowPairs32(b * W, N, low);
-            fieldRows<T, K, W, LDS>(tile, at32, n32, uT, tT, qT, qT1, ST);
-            at32 += n32 * kChunks32 * W;
+            fieldRows<T, K, W, MODE, true>(tile, stream, pj, at, n32, n32, uT, tT, qT, qT1, ST);
+            at += n32 * kChunks32 * W;
 #pragma unroll
             for (int c = 0; c < 6; ++c)
 #pragma unroll
@@ -457,6 +552,7 @@ static __device__ __forceinline__ void fieldAccel(const StepParams& p, const Til
             for (int c = 0; c < 3; ++c)
                 g[k].acc[c] = __fma_rn(cL[k], S[2 * c].v[k], __fma_rn(sL[k], S[2 * c + 1].v[k], g[k].acc[c]));
     }
+    if constexpr (MODE == TileRead::kStream) stream.rewind();
     // fold the set's partial sums of each object
 #pragma unroll
     for (int off = W / 2; off > 0; off >>= 1)

@@ -25,15 +25,17 @@
 // | Xc1 Xs1 | Yc1 Ys1 | Zc1 Zs1) and four in FP32 (A0 A1 Xc0 Xs0 | Yc0 Ys0
 // Zc0 Zs0 | Xc1 Xs1 Yc1 Ys1 | Zc1 Zs1 - -), chunk c of pair i of lane j at
 // ((i chunks + c) W + j): the lanes of a load read consecutive 16-byte words,
-// and a block's pairs follow the block's before.  In split precision the
-// rows of degrees n <= lowDeg + 1 of a column are FP64 pairs, rounded up to
-// whole pairs (by the column alone: the same rows whatever W), and all FP64
-// pairs lie before the FP32 pairs; the one degree more than asked for costs
-// 1.6 % of the rows at degree 70 and keeps the FP32 error below that of the
+// and a block's pairs follow the block's before: the tile is one stream in
+// the order the column loop reads it.  In split precision a block's FP64
+// pairs come first, then its FP32 pairs; the rows of degrees n <= lowDeg + 1
+// of a column are FP64, rounded up to whole pairs (by the column alone: the
+// same rows whatever W).  The one degree more than asked for costs 1.6 % of
+// the rows at degree 70 and keeps the FP32 error below that of the
 // spherical-component sums this form replaced (20,000 LEO objects, 30 steps
 // of 60 s, rms against FP64 at degrees 36 / 70 / 90 / 120: 0.81 / 1.20 / 0.94
 // / 0.96 um; those sums 0.89 / 1.26 / 0.98 / 1.02 um; without the degree 0.90
-// / 1.30 / 1.03 / 1.03 um).
+// / 1.30 / 1.03 / 1.03 um).  The bytes are padded to whole stages of the
+// stream (kStageChunks).
 #pragma once
 #include <vector>
 
@@ -62,10 +64,16 @@ PHOP_GEO_HD int rowPairs32(int M, int N, int lowDeg) {
     return rows > 0 ? (rows + 1) / 2 : 0;
 }
 
+// A tile too large for shared memory is streamed through a ring of
+// kRingStages stages per warp.
+constexpr int kStageChunks = 128;  // 16-byte chunks of a stage: four a lane
+constexpr int kRingStages = 8;
+constexpr int kRingMirror = kChunks64 - 1;  // rows (W <= 8 chunks) repeated past the ring's end
+constexpr int kRingBytes = (kRingStages * kStageChunks + kRingMirror * 8) * 16;
+
 struct HostTile {
     std::vector<unsigned char> bytes;
     int nblocks = 0;
-    int chunk32 = 0;  // 16-byte chunks of FP64 rows before the FP32 rows
 };
 
 struct HostEnvironment;

@@ -87,12 +87,12 @@ struct StepParams {
     const void* tile;       // tile entries in global memory
     int tileBytes;          // multiple of 16
     int nblocks;            // blocks of columns
-    int chunk32;            // split precision: 16-byte chunks of FP64 rows before the FP32 rows
     int lowDeg;             // split precision: FP64 low part
     const void* tile64;     // split precision: the FP64 tile (global memory) of L lanes
     int nblocks64;
     double splitRadius;     // split precision: radius (km) below which the tile part stays FP64; 0 = none
     int useSmemTile;
+    int streamTile;         // the tile streamed through rings in shared memory (hasStream shapes)
     int pairSh;             // the geopotential of lane-group pairs (tile built for 2L lanes)
     int deepRegs;           // host-side choice of the kernel's thread bound (stepThreadBound)
     int tileWaitTest;       // test of the staging time-out: arm the barrier, issue no copy
@@ -116,6 +116,10 @@ __host__ __device__ constexpr int maxStepThreads(int lanes) {
 }
 constexpr int kDeepThreads = 256;
 __host__ __device__ constexpr bool hasDeepShape(int lanes) { return lanes == 2 || lanes == 4; }
+// shapes that read shared memory by their own loads and can stream a tile
+__host__ __device__ constexpr bool hasStream(int lanes, int deep) {
+    return lanes == 1 || (deep && hasDeepShape(lanes));
+}
 __host__ __device__ constexpr int stepThreadBound(int lanes, int deep) {
     return deep && hasDeepShape(lanes) ? kDeepThreads : maxStepThreads(lanes);
 }
@@ -126,10 +130,10 @@ void launchRecordPairs(const EpochRecord* grid, int64_t count, double2* pairs, c
 cudaError_t launchPropagate(const StepParams& p, int lanes, bool split, bool shared, int ctas, int threads,
                             cudaStream_t stream);
 int propagateSmemBytes(const StepParams& p, int lanes, int threads);
-int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int threads, int smem);
+int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int threads, int smem);
 // The compiled instantiation's attributes (maxThreadsPerBlock, numRegs,
 // localSizeBytes): the launch shape never asks for more threads than the
 // instantiation accepts.
-cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, cudaFuncAttributes* a);
+cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, cudaFuncAttributes* a);
 
 }  // namespace phop

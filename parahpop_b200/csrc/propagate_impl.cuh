@@ -421,9 +421,9 @@ static __device__ __noinline__ void tideAloneAccel(const Rec r, const double pos
 // full right-hand side acceleration (km/s^2); every lane of the group calls it.
 // PAIR: two lane groups share their columns (a separate kernel instantiation,
 // so the one-object-per-lane kernel keeps its own register allocation).
-template <int L, typename T, bool PAIR, bool LDS, class Rec>
+template <int L, typename T, bool PAIR, TileRead MODE, class Rec>
 static __device__ __forceinline__ void accelerations(const StepParams& p, const TileRef& tile,
-                                              const Rec& r, const double pos[3], const double vel[3],
+                                              TileStream<(PAIR ? 2 : 1) * L>& stream, const Rec& r, const double pos[3], const double vel[3],
                                               double bc, double ams, double acc[3]) {
     const DevEnv& e = p.env;
     double ax = 0.0, ay = 0.0, az = 0.0;
@@ -473,10 +473,12 @@ static __device__ __forceinline__ void accelerations(const StepParams& p, const 
             // split precision with a floor: objects below the split radius
             // keep every row in FP64 (from the FP64 tile in global memory)
             if (!PAIR && sizeof(T) == 4 && p.splitRadius > 0.0
-                && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius)
-                fieldAccel<L, 1, double, false>(p, TileRef{p.tile64, p.nblocks64, 0, false}, r, bx, by, bz, a);
-            else
-                fieldAccel<L, PAIR ? 2 : 1, T, LDS>(p, tile, r, bx, by, bz, a);
+                && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius) {
+                TileStream<L> none;
+                fieldAccel<L, 1, double, TileRead::kGeneric>(p, TileRef{p.tile64, p.nblocks64, false}, none, r, bx, by, bz, a);
+            } else {
+                fieldAccel<L, PAIR ? 2 : 1, T, MODE>(p, tile, stream, r, bx, by, bz, a);
+            }
             double ai[3];
             if (isEarth) {
                 fromBody(r, a, ai);
@@ -698,22 +700,31 @@ static __device__ __forceinline__ RecordInterp recordFromGrid(const StepParams& 
 // MAXT: the thread bound the kernel is compiled for, which sets its register
 // budget (the register file is split over the SM's four sub-partitions, so
 // 320 or 384 threads leave 168 registers a thread and 256 threads leave 255).
-template <int L, typename T, bool SHARED_GRID, bool PAIR, int MAXT>
+// STREAM: the tile streamed through rings (TileStream).
+template <int L, typename T, bool SHARED_GRID, bool PAIR, int MAXT, bool STREAM>
 __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant__ StepParams p) {
+    constexpr TileRead MODE = STREAM                ? TileRead::kStream
+                              : MAXT <= kDeepThreads ? TileRead::kShared
+                                                     : TileRead::kGeneric;
     constexpr int NA = Axes<L>::N;
-    TileRef tile{p.tile, p.nblocks, p.chunk32, false};
+    TileRef tile{p.tile, p.nblocks, false};
     int kOffset = 0;
     if (!SHARED_GRID && !p.gridPairs) {  // per-object time needs the batch's record grid
         if (threadIdx.x == 0) atomicExch(p.errorFlag, 3);
         return;
     }
-    if (p.useSmemTile) {
+    if (!STREAM && p.useSmemTile) {
         const bool test = p.tileWaitTest != 0;
         if (stageTile(g_smem, p.tile, p.tileBytes, !test, test ? 4096L : (1L << 24)))
             tile.staged = true;
         else if (threadIdx.x == 0 && p.tileFallbacks)
             atomicAdd(p.tileFallbacks, 1);  // this CTA reads the tile from global memory
         kOffset = p.tileBytes;
+    }
+    TileStream<(PAIR ? 2 : 1) * L> stream;
+    if constexpr (STREAM) {
+        stream.begin((int)(threadIdx.x / 32) * kRingBytes, p.tile, p.tileBytes);
+        kOffset = (int)(blockDim.x / 32) * kRingBytes;
     }
     const StageStore kst{(double*)(g_smem + kOffset) + threadIdx.x / L, (int)blockDim.x / L};
     const int lane = (int)(threadIdx.x & 31);
@@ -799,11 +810,11 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
                 }
                 if (SHARED_GRID) {
                     const RecordRef rec{p.records + kstep * 13 + s};
-                    accelerations<L, T, PAIR, MAXT <= kDeepThreads>(p, tile, rec, st, st + 3, bc, ams, acc);
+                    accelerations<L, T, PAIR, MODE>(p, tile, stream, rec, st, st + 3, bc, ams, acc);
                 } else {
                     const double ts = s == 0 ? t0 : t0 + dt * rkC(s - 1);
                     const RecordInterp rec = recordFromGrid(p, ts);
-                    accelerations<L, T, PAIR, MAXT <= kDeepThreads>(p, tile, rec, st, st + 3, bc, ams, acc);
+                    accelerations<L, T, PAIR, MODE>(p, tile, stream, rec, st, st + 3, bc, ams, acc);
                 }
                 if (s < 12) {
 #pragma unroll
@@ -853,6 +864,7 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
             }
         }
     }
+    if constexpr (STREAM) stream.end();
 }
 
 }  // namespace phop

@@ -21,9 +21,11 @@
 
 namespace phop {
 
-// one compiled step-kernel shape: lanes per object, lane-group pairs, thread bound
-template <int L_, bool PAIR_, int MAXT_>
+// one compiled step-kernel shape: lanes per object, lane-group pairs, thread
+// bound, the tile streamed through rings
+template <int L_, bool PAIR_, int MAXT_, bool STREAM_ = false>
 struct Shape {
+    static constexpr bool STREAM = STREAM_;
     static constexpr int L = L_;
     static constexpr bool PAIR = PAIR_;
     static constexpr int MAXT = MAXT_;
@@ -31,9 +33,16 @@ struct Shape {
 
 // The instantiated shapes: 1, 2, 4, 8, 16 lanes at the wide thread bound;
 // pairs at 1, 2, 4 lanes (slower at 8 and 16); the deep bound at 2 and 4
-// lanes, paired or not.  Anything else returns `bad`.
+// lanes, paired or not; a streamed tile at those and at one lane.  Anything
+// else returns `bad`.
 template <class R, class F>
-static R dispatch(int lanes, int pair, int deep, R bad, F&& f) {
+static R dispatch(int lanes, int pair, int deep, int stream, R bad, F&& f) {
+    if (stream) {
+        if (!hasStream(lanes, deep)) return bad;
+        if (lanes == 1) return pair ? f(Shape<1, true, maxStepThreads(1), true>{}) : f(Shape<1, false, maxStepThreads(1), true>{});
+        if (lanes == 2) return pair ? f(Shape<2, true, kDeepThreads, true>{}) : f(Shape<2, false, kDeepThreads, true>{});
+        return pair ? f(Shape<4, true, kDeepThreads, true>{}) : f(Shape<4, false, kDeepThreads, true>{});
+    }
     if (deep && hasDeepShape(lanes)) {
         if (lanes == 2) return pair ? f(Shape<2, true, kDeepThreads>{}) : f(Shape<2, false, kDeepThreads>{});
         return pair ? f(Shape<4, true, kDeepThreads>{}) : f(Shape<4, false, kDeepThreads>{});
@@ -59,13 +68,13 @@ static R dispatch(int lanes, int pair, int deep, R bad, F&& f) {
 
 template <class S>
 static auto kernelOf() {
-    return propagateKernel<S::L, PHOP_T, (bool)PHOP_SG, S::PAIR, S::MAXT>;
+    return propagateKernel<S::L, PHOP_T, (bool)PHOP_SG, S::PAIR, S::MAXT, S::STREAM>;
 }
 
 cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t paramsBytes, int lanes, int ctas,
                                                     int threads, int smem, cudaStream_t stream) {
     if (paramsBytes != sizeof(StepParams)) return cudaErrorInvalidValue;  // objects built from different headers
-    return dispatch(lanes, p.pairSh, p.deepRegs, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
+    return dispatch(lanes, p.pairSh, p.deepRegs, p.streamTile, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
         auto k = kernelOf<decltype(shape)>();
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -76,8 +85,8 @@ cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t 
     });
 }
 
-int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int threads, int smem) {
-    return dispatch(lanes, pair, deep, 0, [&](auto shape) -> int {
+int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int threads, int smem) {
+    return dispatch(lanes, pair, deep, stream, 0, [&](auto shape) -> int {
         auto k = kernelOf<decltype(shape)>();
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int n = 0;
@@ -86,8 +95,8 @@ int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int threads
     });
 }
 
-cudaError_t PHOP_CAT(attributes_, PHOP_SUFFIX)(int lanes, int pair, int deep, cudaFuncAttributes* a) {
-    return dispatch(lanes, pair, deep, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
+cudaError_t PHOP_CAT(attributes_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, cudaFuncAttributes* a) {
+    return dispatch(lanes, pair, deep, stream, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
         return cudaFuncGetAttributes(a, kernelOf<decltype(shape)>());
     });
 }

@@ -156,3 +156,29 @@ def test_field_on_the_polar_axis(tmp_path):
     assert np.isfinite(out).all()
     assert np.abs(out[0] - out[1]).max() <= 2e-9
     p.close()
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("degree", [92, 120])
+def test_streamed_tile_matches_global_reads(tmp_path, degree, split):
+    """A tile that does not fit shared memory is streamed through rings (at
+    degree 92 in split precision it fits and is staged); with "tile_smem" 0
+    the same rows are read from global memory.  The same sums, so the same
+    bits, on a shared time grid and on per-object epochs."""
+    d = S.write_environment(tmp_path, S.EnvSpec(degree=degree))
+    (d / "config.json").write_text(json.dumps(S.make_config(d, 240.0, 60.0, degree=degree)))
+    pop = S.population_leo(99, seed=11)
+    args = (pop.states, pop.mass, pop.drag_area, pop.srp_area, pop.cd, pop.cr)
+    for lanes, pair, deep in ((1, 0, 0), (1, 1, 0), (2, 0, 1), (2, 1, 1), (4, 0, 1), (4, 1, 1)):
+        p = api.Propagator(d / "config.json", lanes=lanes, split=split)
+        p.set_option("pair_sh", pair)
+        p.set_option("deep_registers", deep)
+        for epochs in (pop.epochs, pop.epochs + np.linspace(0.0, 0.01, len(pop))):
+            got = []
+            for staged in (1, 0):
+                p.set_option("tile_smem", staged)
+                got.append(p.propagate(epochs, *args)[1])
+                assert p.stats()["tile_in_smem"] == (1 if staged and split and degree == 92 else 0)
+            assert np.isfinite(got[0]).all()
+            np.testing.assert_array_equal(got[0], got[1])
+        p.close()
