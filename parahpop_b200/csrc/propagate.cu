@@ -18,14 +18,21 @@ PHOP_DECL(f32_grid)
 PHOP_DECL(f32_mixed)
 #undef PHOP_DECL
 
-// One epoch record per thread; then the warp forms the tide corrections of
-// its records one after the other, the terms split across its lanes
-// (tidefield::tideDeltasWarp: lane s < 25 owns coefficient slot s).
+// A warp takes `per` records: the first `per` lanes evaluate one each, then
+// the whole warp forms their tide corrections one after the other, the terms
+// split across its lanes (tidefield::tideDeltasWarp: lane s < 25 owns
+// coefficient slot s).  The corrections are a serial chain of several
+// thousand cycles a record, so few records (a uniform batch has 13 a step)
+// are spread over as many warps as there are: 130 records in full force took
+// 0.35 ms at 32 a warp, 0.07 at one; a grid of tens of thousands takes
+// 32 a warp, where every lane has a record of its own to evaluate.
 __global__ void __launch_bounds__(64) epochRecordsKernel(const __grid_constant__ DevEnv env,
-                                                         const double* __restrict__ epochs, int count,
+                                                         const double* __restrict__ epochs, int count, int per,
                                                          EpochRecord* __restrict__ out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = i < count;
+    const int lane = threadIdx.x & 31;
+    const int first = (int)((blockIdx.x * blockDim.x + threadIdx.x) / 32) * per;
+    const int i = first + lane;
+    const bool live = lane < per && i < count;
     tidefield::Epoch tin;
     bool tides = false;
     if (live) {
@@ -35,8 +42,6 @@ __global__ void __launch_bounds__(64) epochRecordsKernel(const __grid_constant__
     }
     if (!(env.solid || env.ocean)) return;
     __syncwarp();
-    const int lane = threadIdx.x & 31;
-    const int warpFirst = i - lane;
     unsigned todo = __ballot_sync(0xffffffffu, tides);
     while (todo) {
         const int src = __ffs(todo) - 1;
@@ -56,8 +61,8 @@ __global__ void __launch_bounds__(64) epochRecordsKernel(const __grid_constant__
         tidefield::tideDeltasWarp(ep, env.solid != 0, env.ocean != 0, env.zeroTide != 0, env.tideOcean,
                                   env.tideScale, dC, dS);
         if (lane < tidefield::kSlots) {
-            out[warpFirst + src].dC[lane + 3] = dC * env.tideNorm[lane];
-            out[warpFirst + src].dS[lane + 3] = dS * env.tideNorm[lane];
+            out[first + src].dC[lane + 3] = dC * env.tideNorm[lane];
+            out[first + src].dS[lane + 3] = dS * env.tideNorm[lane];
         }
     }
 }
@@ -65,7 +70,11 @@ __global__ void __launch_bounds__(64) epochRecordsKernel(const __grid_constant__
 void launchEpochRecords(const DevEnv& env, const double* epochs, int count, EpochRecord* out, cudaStream_t stream) {
     if (count <= 0) return;
     const int threads = 64;
-    epochRecordsKernel<<<(count + threads - 1) / threads, threads, 0, stream>>>(env, epochs, count, out);
+    // up to eight warps an SM, then more records a warp
+    const int kWarps = 148 * 8;
+    const int per = count <= kWarps ? 1 : count >= 32 * kWarps ? 32 : (count + kWarps - 1) / kWarps;
+    const int warps = (count + per - 1) / per;
+    epochRecordsKernel<<<(warps * 32 + threads - 1) / threads, threads, 0, stream>>>(env, epochs, count, per, out);
 }
 
 static __global__ void recordPairsKernel(const EpochRecord* __restrict__ grid, int64_t total, double2* __restrict__ pairs) {
