@@ -1060,11 +1060,14 @@ Engine::Engine(const HostEnvironment& env, int device) : host_(env), serial_(++g
     PHOP_CUDA(cudaSetDevice(device_));
     PHOP_CUDA(cudaDeviceGetAttribute(&sms_, cudaDevAttrMultiProcessorCount, device_));
     PHOP_CUDA(cudaDeviceGetAttribute(&maxSmem_, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+    for (cudaEvent_t& e : events_) PHOP_CUDA(cudaEventCreate(&e));
     uploadEnvironment();
 }
 
 Engine::~Engine() {
     cudaSetDevice(device_);
+    for (cudaEvent_t e : events_)
+        if (e) cudaEventDestroy(e);
     for (void* p : owned_) cudaFree(p);
     for (auto& kv : scratch_) cudaFree(kv.second.first);
     for (GraphEntry& g : graphs_) cudaGraphExecDestroy(g.exec);
@@ -1695,28 +1698,25 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
     p.gridN = g.gridN;
     p.stride = g.stride;
     const bool shared = g.shared;
-    cudaEvent_t e0, e1, e2, eTuned;
-    PHOP_CUDA(cudaEventCreate(&e0));
-    PHOP_CUDA(cudaEventCreate(&e1));
-    PHOP_CUDA(cudaEventCreate(&e2));
-    PHOP_CUDA(cudaEventCreate(&eTuned));
+    const cudaEvent_t e0 = events_[0], e1 = events_[1], e2 = events_[2], eTuned = events_[3];
     int64_t launches = launchesBefore;
     PHOP_CUDA(cudaEventRecord(e0, stream));
     if (shared) {
         const int nsteps = (int)g.t0.size();
-        std::vector<double> stageT((size_t)nsteps * 13);
+        // step starts, step sizes and stage epochs in one buffer and one copy
+        std::vector<double> times((size_t)nsteps * 15);
+        std::copy(g.t0.begin(), g.t0.end(), times.begin());
+        std::copy(g.dt.begin(), g.dt.end(), times.begin() + nsteps);
+        double* stageT = times.data() + (size_t)nsteps * 2;
         static const double c[12] = {2. / 27, 1. / 9, 1. / 6, 5. / 12, 1. / 2, 5. / 6, 1. / 6, 2. / 3, 1. / 3, 1.0, 0, 1.0};
         for (int k = 0; k < nsteps; ++k)
             for (int s = 0; s < 13; ++s)
                 stageT[(size_t)k * 13 + s] = s == 0 ? g.t0[k] : std::fma(g.dt[k], c[s - 1], g.t0[k]);
-        double* dStage = (double*)scratch("stageT", stageT.size() * sizeof(double));
-        EpochRecord* dRec = (EpochRecord*)scratch("records", stageT.size() * sizeof(EpochRecord));
-        double* dT0 = (double*)scratch("t0", (size_t)nsteps * sizeof(double));
-        double* dDtv = (double*)scratch("dt", (size_t)nsteps * sizeof(double));
-        PHOP_CUDA(cudaMemcpyAsync(dStage, stageT.data(), stageT.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
-        PHOP_CUDA(cudaMemcpyAsync(dT0, g.t0.data(), (size_t)nsteps * sizeof(double), cudaMemcpyHostToDevice, stream));
-        PHOP_CUDA(cudaMemcpyAsync(dDtv, g.dt.data(), (size_t)nsteps * sizeof(double), cudaMemcpyHostToDevice, stream));
-        launchEpochRecords(denv_, dStage, (int)stageT.size(), dRec, stream);
+        double* dT0 = (double*)scratch("times", times.size() * sizeof(double));
+        double *dDtv = dT0 + nsteps, *dStage = dT0 + (size_t)2 * nsteps;
+        EpochRecord* dRec = (EpochRecord*)scratch("records", (size_t)nsteps * 13 * sizeof(EpochRecord));
+        PHOP_CUDA(cudaMemcpyAsync(dT0, times.data(), times.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
+        launchEpochRecords(denv_, dStage, nsteps * 13, dRec, stream);
         PHOP_CUDA(cudaGetLastError());
         ++launches;
         p.nsteps = nsteps;
@@ -1777,10 +1777,6 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
         stats->deepRegs = p.deepRegs != 0;
         stats->registers = shape.registers;
     }
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    cudaEventDestroy(e2);
-    cudaEventDestroy(eTuned);
 }
 
 // time grid of one object (FixedStep.h:7-37): step start epochs and sizes
@@ -1812,11 +1808,11 @@ void Engine::propagate(const TargetSet& t, int64_t maxSteps, const RunOptions& o
     PHOP_CUDA(cudaSetDevice(device_));
     const int64_t n = (int64_t)t.size();
     if (n == 0) throw std::runtime_error("targets must be a nonempty array.");
-    cudaEvent_t a0, a1;
-    PHOP_CUDA(cudaEventCreate(&a0));
-    PHOP_CUDA(cudaEventCreate(&a1));
+    const cudaEvent_t a0 = events_[4], a1 = events_[5];
     PHOP_CUDA(cudaEventRecord(a0, stream));
-    std::vector<double> soa((size_t)6 * n), bc(n), ams(n);
+    // states (6 x n), drag and radiation factors in one buffer and one copy
+    std::vector<double> soa((size_t)8 * n);
+    double *bc = soa.data() + (size_t)6 * n, *ams = soa.data() + (size_t)7 * n;
     for (int64_t i = 0; i < n; ++i) {
         for (int d = 0; d < 6; ++d) soa[(size_t)d * n + i] = t.state[(size_t)6 * i + d];
         // driver.cpp:118-120 then PrivateAccelerations.h:41-42
@@ -1826,11 +1822,8 @@ void Engine::propagate(const TargetSet& t, int64_t maxSteps, const RunOptions& o
         bc[i] = t.cd[i] * area / t.mass[i];
     }
     double* dState = (double*)scratch("state", soa.size() * sizeof(double));
-    double* dBc = (double*)scratch("bc", (size_t)n * sizeof(double));
-    double* dAms = (double*)scratch("ams", (size_t)n * sizeof(double));
+    const double *dBc = dState + (size_t)6 * n, *dAms = dState + (size_t)7 * n;
     PHOP_CUDA(cudaMemcpyAsync(dState, soa.data(), soa.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
-    PHOP_CUDA(cudaMemcpyAsync(dBc, bc.data(), bc.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
-    PHOP_CUDA(cudaMemcpyAsync(dAms, ams.data(), ams.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
     bool uniform = true;
     for (int64_t i = 1; i < n && uniform; ++i)
         uniform = t.epoch[i] == t.epoch[0] && t.duration[i] == t.duration[0] && t.step[i] == t.step[0];
@@ -1847,7 +1840,7 @@ void Engine::propagate(const TargetSet& t, int64_t maxSteps, const RunOptions& o
         g.t0 = std::move(t0);
         g.dt = std::move(dt);
         int64_t launches = 0;
-        const int64_t* dOrder = opt.ordered ? orderByRadius(n, dState, stream, &launches) : nullptr;
+        const int64_t* dOrder = ordersObjects(opt) ? orderByRadius(n, dState, stream, &launches) : nullptr;
         runKernel(n, dState, dBc, dAms, g, dOrder, maxSteps, opt, st, stream, launches);
         std::fill(outEpoch.begin(), outEpoch.end(), etToMjdHost(finalEt));
         st->objectSteps += n * (int64_t)g.t0.size();
@@ -1921,14 +1914,12 @@ void Engine::propagate(const TargetSet& t, int64_t maxSteps, const RunOptions& o
             outEpoch[i] = etToMjdHost(cur[i]);
         }
     }
-    PHOP_CUDA(cudaMemcpyAsync(soa.data(), dState, soa.size() * sizeof(double), cudaMemcpyDeviceToHost, stream));
+    PHOP_CUDA(cudaMemcpyAsync(soa.data(), dState, (size_t)6 * n * sizeof(double), cudaMemcpyDeviceToHost, stream));
     PHOP_CUDA(cudaEventRecord(a1, stream));
     PHOP_CUDA(cudaEventSynchronize(a1));
     float ms = 0;
     cudaEventElapsedTime(&ms, a0, a1);
     st->totalMs += ms;
-    cudaEventDestroy(a0);
-    cudaEventDestroy(a1);
     outState.assign((size_t)6 * n, 0.0);
     for (int64_t i = 0; i < n; ++i)
         for (int d = 0; d < 6; ++d) outState[(size_t)6 * i + d] = soa[(size_t)d * n + i];
@@ -2016,7 +2007,7 @@ int64_t Engine::advanceObjects(int64_t n, double* dState, double* dTime, const d
     g.unfinished = (int*)scratch("unfinished", (size_t)n * 4);
     int64_t launches = 1;  // the span kernel
     buildRecordGrid(lo, hi, g, stream, &launches);
-    const int64_t* dOrder = opt.ordered ? orderByRadius(n, dState, stream, &launches) : nullptr;
+    const int64_t* dOrder = ordersObjects(opt) ? orderByRadius(n, dState, stream, &launches) : nullptr;
     RunOptions o = opt;
     o.graph = false;  // every slice's launch parameters differ: nothing to replay
     runKernel(n, dState, dBc, dAms, g, dOrder, maxSteps, o, st, stream, launches);
@@ -2049,7 +2040,7 @@ void Engine::propagateResident(int64_t n, double* dState, const double* epochMjd
     g.t0 = std::move(t0);
     g.dt = std::move(dt);
     int64_t launches = 0;
-    const int64_t* dOrder = opt.ordered ? orderByRadius(n, dState, stream, &launches) : nullptr;
+    const int64_t* dOrder = ordersObjects(opt) ? orderByRadius(n, dState, stream, &launches) : nullptr;
     runKernel(n, dState, dBc, dAms, g, dOrder, maxSteps, opt, st, stream, launches);
     st->objectSteps += n * nsteps;
     outEpochMjd.assign(n, etToMjdHost(finalEt));

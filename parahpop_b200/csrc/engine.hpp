@@ -240,6 +240,9 @@ private:
     // stride `stride`); `slots` (nullable) lists the objects to order
     const int64_t* orderByRadius(int64_t n, const double* dState, cudaStream_t stream, int64_t* launches,
                                  int64_t stride = 0, const int64_t* slots = nullptr);
+    // The order only keeps warps together in the NRLMSISE-00 branches: without
+    // that model the sort (a key kernel and six of CUB's) would buy nothing.
+    bool ordersObjects(const RunOptions& opt) const { return opt.ordered && denv_.hasNrl; }
     void buildRecordGrid(double lo, double hi, TimeGrid& g, cudaStream_t stream, int64_t* launches);
     LaunchShape launchStep(StepParams p, int lanes, const RunOptions& opt, bool shared, cudaStream_t stream);
     LaunchShape prepareStep(StepParams& p, int lanes, const RunOptions& opt, bool shared);
@@ -258,6 +261,7 @@ private:
     double2* pairCache_ = nullptr;  // gridCache_ as value pairs (StepParams::gridPairs)
     int64_t gridKLo_ = 0, gridKHi_ = -1;
     cudaStream_t captureStream_ = nullptr;
+    cudaEvent_t events_[6] = {};  // timing marks of one call (a context serves one call at a time)
     // autotuned launch shape of a batch class: lanes * 2 + (pairs ? 1 : 0)
     int tunedShape(const StepParams& base, const RunOptions& opt, bool shared, cudaStream_t stream, int64_t* launches);
     void runKernel(int64_t n, double* dState, const double* dBc, const double* dAms, const TimeGrid& g,
