@@ -398,6 +398,24 @@ struct NrlMeso {
     T dm28;
 };
 
+// Sines and cosines of the model's geodetic latitude and longitude, whose
+// degrees it turns to radians by the rounded factor 1.74533e-2: from those of
+// the true angles by the small rotation the factor's excess makes
+// (4.3e-7 of the angle), which costs a few products where sincos of each costs
+// several hundred cycles.
+template <typename T>
+struct Angles {
+    T sLat, cLat, sLon, cLon;
+    static __device__ __forceinline__ void turn(T s, T c, T angle, T& so, T& co) {
+        const T e = angle * T(1.74533E-2 * 57.2957795130823208768 - 1.0);
+        const T h = T(1.0) - T(0.5) * e * e;
+        so = s * h + c * e;
+        co = c * h - s * e;
+    }
+    __device__ __forceinline__ void latitude(T s, T c, T angle) { turn(s, c, angle, sLat, cLat); }
+    __device__ __forceinline__ void longitude(T s, T c, T angle) { turn(s, c, angle, sLon, cLon); }
+};
+
 // Per-object part.  Returns the gtd7d total mass density in kg/m^3.
 template <typename T>
 struct Fast {
@@ -419,10 +437,9 @@ struct Fast {
 
     __device__ __forceinline__ T zeta(T zz, T zl) const { return (zz - zl) * (re + zl) * rcp(re + zz); }
 
-    __device__ __forceinline__ void basis(T lat, T lst) {
-        const T dgtr = T(1.74533E-2), hr = T(0.2618);
-        T c, s;
-        sincos(lat * dgtr, &c, &s);  // c = sin(lat), s = cos(lat)
+    __device__ __forceinline__ void basis(const Angles<T>& a, T lst) {
+        const T hr = T(0.2618);
+        const T c = a.sLat, s = a.cLat;
         const T c2 = c * c, c4 = c2 * c2, s2 = s * s;
         plg[0][1] = c;
         plg[0][2] = T(0.5) * (T(3.0) * c2 - T(1.0));
@@ -453,7 +470,8 @@ struct Fast {
         c2tloc = (ctloc - stloc) * (ctloc + stloc);
         s3tloc = stloc * (T(3.0) - T(4.0) * stloc * stloc);
         c3tloc = ctloc * (T(4.0) * ctloc * ctloc - T(3.0));
-        sincos(dgtr * gLong, &sgl, &cgl);
+        sgl = a.sLon;
+        cgl = a.cLon;
         s2gl = T(2.0) * sgl * cgl;
         c2gl = (cgl - sgl) * (cgl + sgl);
     }
@@ -824,11 +842,14 @@ struct Fast {
         // alternates this model with the geopotential loop, and both compete
         // for the instruction cache; measured 1-2 % faster on the uneven
         // population at two lanes than the fully unrolled form, which the
-        // eight- and sixteen-lane kernels keep: they call the model out of line)
+        // eight- and sixteen-lane kernels keep: they call the model out of
+        // line), four pairs an iteration so that their reads overlap (one
+        // warp at four lanes 15.5 -> 14.2, at one lane 23.2 -> 21.0 thousand
+        // cycles a density above 450 km)
         T mono[kGlobeBasis + 1];
 #pragma unroll
         for (int i = 0; i <= kGlobeBasis; ++i) mono[i] = globeMonomial(i, x, x2, U1, U2);
-#pragma unroll 1
+#pragma unroll 4
         for (int i = 0; i < kGlobeBasis; i += 2) {
             const T b0 = mono[i], b1 = mono[i + 1];
 #pragma unroll
@@ -1130,6 +1151,13 @@ struct Fast {
     // lanes starting at groupBase (all lanes of the group get the result)
     template <int L>
     __device__ __forceinline__ T density(T lat, T lon, T alt, T lst, int j, int groupBase) {
+        Angles<T> a;
+        sincos(lat * T(1.74533E-2), &a.sLat, &a.cLat);
+        sincos(lon * T(1.74533E-2), &a.sLon, &a.cLon);
+        return density<L>(lat, lon, alt, lst, a, j, groupBase);
+    }
+    template <int L>
+    __device__ __forceinline__ T density(T lat, T lon, T alt, T lst, const Angles<T>& ang, int j, int groupBase) {
         glat = lat;
         absLat = fabs(lat);
         gLong = lon;
@@ -1139,10 +1167,10 @@ struct Fast {
         ms.tn1[0] = T(0);
         ms.tgn1[0] = T(0);
         // glatf
-        const T c2 = cos(T(2.0) * T(1.74533E-2) * lat);
+        const T c2 = T(1.0) - T(2.0) * ang.sLat * ang.sLat;  // cos of twice the latitude
         gsurf = T(980.616) * (T(1.0) - T(0.0026373) * c2);
         re = T(2.0) * gsurf * rcp(T(3.085462E-6) + T(2.27E-9) * c2) * T(1.0E-5);
-        basis(lat, lst);
+        basis(ang, lst);
         T G[kGlobeTasks];
         T aptTlb = T(0), aptLast = T(0);
         globeTasks<L>(G, aptTlb, aptLast, j, groupBase);
