@@ -1095,6 +1095,7 @@ void Engine::uploadEnvironment() {
         e.tideScale[n] = h.hasShape && h.shBodyId == 399
                              ? (tidefield::kMuEarth * 1e-9 / h.shGM) * std::pow(tidefield::kRadius * 1e-3 / h.shR, (double)n)
                              : 1.0;
+    columns_ = h.hasShape ? fieldOrder(h) + 2 : 0;
     const bool joined = h.hasShape && h.shBodyId == 399;
     for (int slot = 0; slot < tidefield::kSlots; ++slot) {
         int n, m;
@@ -1513,8 +1514,14 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     }
     // shared memory per CTA: the coefficient tile (when it fits) plus the
     // stage accelerations of its objects
-    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - bytes) / kStageBytes * L / 32 * 32; };
-    const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs));
+    // warps in pairs: half of a CTA's warps hold objects; the static mail of
+    // the pairs takes some shared memory
+    p.duo = opt.duo && hasDuo(L, p.pairSh) && (opt.threads <= 0 || opt.threads >= 64) && denv_.hasNrl && (denv_.bodyFlags[denv_.earthIndex] & kAtmosphere)
+            && p.splitRadius == 0.0;
+    const int halves = p.duo ? 2 : 1;
+    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - (p.duo ? 4096 : 0) - bytes) / kStageBytes * L / 32 * 32 * halves; };
+    const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
+                      * (32 * halves);
     const int staged = opt.tileSmem != 0 && tile.bytes + 1024 <= maxSmem_ ? fit(tile.bytes) : 0;
     p.useSmemTile = staged >= 64;
     // A tile that does not fit, or leaves room for fewer than three quarters
@@ -1522,8 +1529,8 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     // can (a streamed row costs about a fifth more than a staged one);
     // "tile_smem" = 0 asks for reads through L1, and the FP64 floor of the
     // split form lets a warp's objects part in the row loop.
-    const int streamed = (maxSmem_ - 1024) / (kRingBytes + kStageBytes * (32 / L)) * 32;
-    p.streamTile = opt.tileSmem != 0 && hasStream(L, p.deepRegs) && tile.nblocks > 0 && p.splitRadius == 0.0
+    const int streamed = (maxSmem_ - 1024 - (p.duo ? 4096 : 0)) / (kRingBytes + kStageBytes * (32 / L)) * 32 * halves;
+    p.streamTile = opt.tileSmem != 0 && (p.duo ? L <= 4 : hasStream(L, p.deepRegs)) && tile.nblocks > 0 && p.splitRadius == 0.0
                    && std::min(staged, bound) < std::min(streamed, bound) * 3 / 4;
     if (p.streamTile) p.useSmemTile = 0;
     int registers = 0;
@@ -1532,14 +1539,14 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
         // never more threads than the compiled instantiation accepts (its
         // register count times the threads must fit the SM's register file)
         const int akey = ((((L * 2 + (opt.split ? 1 : 0)) * 2 + (shared ? 1 : 0)) * 2 + p.pairSh) * 2 + p.deepRegs) * 2
-                         + p.streamTile;
+                         + p.streamTile + 4096 * p.duo;
         auto at = attrs_.find(akey);
         if (at == attrs_.end()) {
             cudaFuncAttributes a{};
-            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, &a));
+            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, p.duo, &a));
             at = attrs_.emplace(akey, std::make_pair(a.maxThreadsPerBlock, a.numRegs)).first;
         }
-        threadsReq = std::max(32, std::min(threadsReq, at->second.first / 32 * 32));
+        threadsReq = std::max(32 * halves, std::min(threadsReq, at->second.first / (32 * halves) * (32 * halves)));
         registers = at->second.second;
     }
     int threads = std::min(threadsReq, p.useSmemTile ? staged : p.streamTile ? streamed : fit(0));
@@ -1547,12 +1554,12 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     if (perSm <= 0) {
         const int smem = propagateSmemBytes(p, L, threads);
         const int64_t key = (((((int64_t)smem * 1024 + threads) * 32 + L) * 4 + (opt.split ? 2 : 0) + (shared ? 1 : 0)) * 2
-                             + p.pairSh) * 4 + p.deepRegs * 2 + p.streamTile;
+                             + p.pairSh) * 8 + p.duo * 4 + p.deepRegs * 2 + p.streamTile;
         auto it = occupancy_.find(key);
         if (it == occupancy_.end())
             it = occupancy_
-                     .emplace(key, propagateMaxCtasPerSm(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, threads,
-                                                    smem))
+                     .emplace(key, propagateMaxCtasPerSm(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, p.duo,
+                                                    threads, smem))
                      .first;
         perSm = it->second;
     }
@@ -1561,11 +1568,11 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     // spread the warps evenly over all SMs instead of filling CTAs first
     const int64_t warpsNeeded = (p.n + (32 / L) - 1) / (32 / L);
     const int64_t slots = (int64_t)sms_ * perSm;
-    if (warpsNeeded <= slots * (threads / 32)) {
+    if (warpsNeeded <= slots * (threads / (32 * halves))) {
         const int64_t warpsPerCta = (warpsNeeded + slots - 1) / slots;
-        threads = (int)std::min<int64_t>(threads, std::max<int64_t>(1, warpsPerCta) * 32);
+        threads = (int)std::min<int64_t>(threads, std::max<int64_t>(1, warpsPerCta) * 32 * halves);
     }
-    const int64_t warpsPerCta = threads / 32;
+    const int64_t warpsPerCta = threads / (32 * halves);
     const int64_t need = (warpsNeeded + warpsPerCta - 1) / warpsPerCta;
     LaunchShape shape;
     shape.lanes = L;
@@ -1580,7 +1587,8 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
 // objects per lane in the geopotential (one, or two for lane-group pairs at
 // up to four lanes) and, at two and four lanes, the thread bound the kernel
 // is compiled for (wide: 320 / 384 threads at 168 registers; deep: 256
-// threads at 255 registers).  Threads per CTA follow from the bound, shared
+// threads at 255 registers), and for small batches the drag model on a second
+// warp.  Threads per CTA follow from the bound, shared
 // memory and the batch size (prepareStep).  The first batch of each class
 // (log2 of the batch size, time-grid mode, precision, pairing and bound
 // options) times a short probe of
@@ -1602,7 +1610,7 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
     if (base.stride != 0 && base.stride != base.n) {  // pools pin their lane count
         const int L = autoLanes(base.n);
         const int pair = opt.pairSh < 0 ? (L <= 4 ? 1 : 0) : opt.pairSh;
-        return (L * 2 + pair) * 2 + (opt.deepRegs > 0 && hasDeepShape(L) ? 1 : 0);
+        return ((L * 2 + pair) * 2 + (opt.deepRegs > 0 && hasDeepShape(L) ? 1 : 0)) * 2;
     }
     const int64_t n = base.n;
     StepParams p = base;
@@ -1620,22 +1628,30 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
     cudaEvent_t e0, e1;
     PHOP_CUDA(cudaEventCreate(&e0));
     PHOP_CUDA(cudaEventCreate(&e1));
-    int best = (autoLanes(n) * 2 + (opt.pairSh > 0 ? 1 : 0)) * 2;
+    int best = (autoLanes(n) * 2 + (opt.pairSh > 0 ? 1 : 0)) * 4;
     float bestMs = 1e30f;
     const char* logEnv = std::getenv("PARAHPOP_B200_TUNE_LOG");
     const bool tuneLog = logEnv && std::atoi(logEnv) != 0;
-    // shape code: ((lanes * 2 + pairs) * 2 + deep thread bound)
-    for (int code = 4; code < 68; ++code) {
-        const int L = code >> 2, pair = (code >> 1) & 1, deep = code & 1;
+    // shape code: (((lanes * 2 + pairs) * 2 + deep thread bound) * 2 + drag on a second warp)
+    for (int code = 8; code < 136; ++code) {
+        const int L = code >> 3, pair = (code >> 2) & 1, deep = (code >> 1) & 1, duo = code & 1;
         if (L != 1 && L != 2 && L != 4 && L != 8 && L != 16) continue;
         if (opt.pairSh >= 0 && pair != opt.pairSh) continue;
         if (opt.pairSh < 0 && pair && L >= 8) continue;  // pairs at 8 and 16 lanes measured slower on every workload
         if (deep && !hasDeepShape(L)) continue;
         if (opt.deepRegs >= 0 && deep != (opt.deepRegs && hasDeepShape(L) ? 1 : 0)) continue;
         if (L >= 8 && n >= (int64_t)sms_ * 512 * 4) continue;  // enough objects to fill the GPU with narrow groups
+        // without a field there are no columns to share; with more than a few
+        // columns sharing wins up to four lanes, and the deep bound over the
+        // wide one, on every workload: those counterparts are not timed
+        if (opt.pairSh < 0 && L <= 4 && pair && columns_ == 0) continue;
+        if (opt.pairSh < 0 && L <= 4 && !pair && columns_ > 16) continue;
+        if (opt.deepRegs < 0 && hasDeepShape(L) && !deep) continue;
+        if (duo && (!hasDuo(L, pair) || !duoFits(n, L))) continue;
         RunOptions o = opt;
         o.pairSh = pair;
         o.deepRegs = deep;
+        o.duo = duo;
         // an untimed launch first (module loading, attribute set-up), then the
         // fastest of two timed probes
         float ms = 1e30f;
@@ -1661,9 +1677,9 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
         if (err) throw std::runtime_error("Propagation kernel reported error " + std::to_string(err) + ".");
         if (tuneLog)
             std::fprintf(stderr,
-                         "parahpop-b200 tune: n=%lld shared=%d split=%d lanes=%d pairs=%d deep=%d probe_steps=%d "
-                         "probe_ms=%.3f\n",
-                         (long long)n, shared ? 1 : 0, opt.split ? 1 : 0, L, pair, deep, probeSteps, ms);
+                         "parahpop-b200 tune: n=%lld shared=%d split=%d lanes=%d pairs=%d deep=%d duo=%d "
+                         "probe_steps=%d probe_ms=%.3f\n",
+                         (long long)n, shared ? 1 : 0, opt.split ? 1 : 0, L, pair, deep, duo, probeSteps, ms);
         if (ms < bestMs) {
             bestMs = ms;
             best = code;
@@ -1737,9 +1753,10 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
     int L = opt.lanes;
     if (L <= 0) {
         const int code = tunedShape(p, opt, shared, stream, &launches);
-        L = code >> 2;
-        o.pairSh = (code >> 1) & 1;
-        o.deepRegs = code & 1;
+        L = code >> 3;
+        o.pairSh = (code >> 2) & 1;
+        o.deepRegs = (code >> 1) & 1;
+        o.duo = code & 1;
     }
     if (opt.dTraj) {  // after the autotuner's probes, which must not write records
         p.traj = opt.dTraj;

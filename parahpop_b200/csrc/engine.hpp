@@ -149,6 +149,8 @@ struct RunOptions {
                           // -1 autotuned with the lane count (pinned lanes: on up to 4 lanes)
     int deepRegs = -1;    // thread bound at 2 and 4 lanes: 1 deep (256 threads, 255 registers), 0 wide
                           // (320 / 384 threads, 168 registers), -1 autotuned (pinned lanes: wide)
+    int duo = 0;          // small batches: the drag model on a second warp (StepParams::duo); the autotuner's
+                          // choice (pinned lanes: 0)
     // trajectory records of a uniform batch: device buffer of
     // (steps / trajEvery) x 6 x n doubles, null for none
     double* dTraj = nullptr;
@@ -240,6 +242,14 @@ private:
     // stride `stride`); `slots` (nullable) lists the objects to order
     const int64_t* orderByRadius(int64_t n, const double* dState, cudaStream_t stream, int64_t* launches,
                                  int64_t stride = 0, const int64_t* slots = nullptr);
+    // Whether a batch is small enough for the drag model on a second warp:
+    // one wave of main warps (four of a CTA's eight).  Beyond it the idle
+    // partners of objects above the atmosphere and the halved main warps cost
+    // more than the overlap gives (10^4 LEO objects at four lanes, 2.1 waves:
+    // 7.6 -> 11.4 ms a twelve-step probe; 4,000 objects, one wave: 4.8 -> 3.3).
+    bool duoFits(int64_t n, int lanes) const {
+        return denv_.hasNrl && (n * lanes + 31) / 32 <= (int64_t)sms_ * (kDeepThreads / 64);
+    }
     // The order only keeps warps together in the NRLMSISE-00 branches: without
     // that model the sort (a key kernel and six of CUB's) would buy nothing.
     bool ordersObjects(const RunOptions& opt) const { return opt.ordered && denv_.hasNrl; }
@@ -262,7 +272,7 @@ private:
     int64_t gridKLo_ = 0, gridKHi_ = -1;
     cudaStream_t captureStream_ = nullptr;
     cudaEvent_t events_[6] = {};  // timing marks of one call (a context serves one call at a time)
-    // autotuned launch shape of a batch class: lanes * 2 + (pairs ? 1 : 0)
+    // autotuned launch shape of a batch class (the code's bits: tunedShape in engine.cu)
     int tunedShape(const StepParams& base, const RunOptions& opt, bool shared, cudaStream_t stream, int64_t* launches);
     void runKernel(int64_t n, double* dState, const double* dBc, const double* dAms, const TimeGrid& g,
                    const int64_t* dOrder, int64_t maxSteps, const RunOptions& opt, RunStats* stats,
@@ -273,6 +283,7 @@ private:
     int device_ = 0;
     int sms_ = 0;
     int maxSmem_ = 0;
+    int columns_ = 0;  // of the geopotential
     DevEnv denv_{};
     std::vector<void*> owned_;
     std::map<std::string, std::pair<void*, size_t>> scratch_;

@@ -94,6 +94,7 @@ struct StepParams {
     int useSmemTile;
     int streamTile;         // the tile streamed through rings in shared memory (hasStream shapes)
     int pairSh;             // the geopotential of lane-group pairs (tile built for 2L lanes)
+    int duo;                // warps in pairs, the drag model on the second (hasDuo shapes)
     int deepRegs;           // host-side choice of the kernel's thread bound (stepThreadBound)
     int tileWaitTest;       // test of the staging time-out: arm the barrier, issue no copy
     // scheduling and errors
@@ -120,8 +121,12 @@ __host__ __device__ constexpr bool hasDeepShape(int lanes) { return lanes == 2 |
 __host__ __device__ constexpr bool hasStream(int lanes, int deep) {
     return lanes == 1 || (deep && hasDeepShape(lanes));
 }
-__host__ __device__ constexpr int stepThreadBound(int lanes, int deep) {
-    return deep && hasDeepShape(lanes) ? kDeepThreads : maxStepThreads(lanes);
+// shapes with the drag model on a second warp, at the deep bound: two lane
+// groups sharing columns up to four lanes, one object a lane at eight and
+// sixteen
+__host__ __device__ constexpr bool hasDuo(int lanes, int pair) { return lanes >= 8 ? !pair : pair != 0; }
+__host__ __device__ constexpr int stepThreadBound(int lanes, int deep, int duo = 0) {
+    return duo || (deep && hasDeepShape(lanes)) ? kDeepThreads : maxStepThreads(lanes);
 }
 
 void launchEpochRecords(const DevEnv& env, const double* epochs, int count, EpochRecord* out, cudaStream_t stream);
@@ -130,10 +135,10 @@ void launchRecordPairs(const EpochRecord* grid, int64_t count, double2* pairs, c
 cudaError_t launchPropagate(const StepParams& p, int lanes, bool split, bool shared, int ctas, int threads,
                             cudaStream_t stream);
 int propagateSmemBytes(const StepParams& p, int lanes, int threads);
-int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int threads, int smem);
+int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int threads, int smem);
 // The compiled instantiation's attributes (maxThreadsPerBlock, numRegs,
 // localSizeBytes): the launch shape never asks for more threads than the
 // instantiation accepts.
-cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, cudaFuncAttributes* a);
+cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, cudaFuncAttributes* a);
 
 }  // namespace phop

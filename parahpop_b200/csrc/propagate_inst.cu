@@ -22,10 +22,10 @@
 namespace phop {
 
 // one compiled step-kernel shape: lanes per object, lane-group pairs, thread
-// bound, the tile streamed through rings
-template <int L_, bool PAIR_, int MAXT_, bool STREAM_ = false>
+// bound, the tile streamed through rings, the drag model on a second warp
+template <int L_, bool PAIR_, int MAXT_, bool STREAM_ = false, bool DUO_ = false>
 struct Shape {
-    static constexpr bool STREAM = STREAM_;
+    static constexpr bool STREAM = STREAM_, DUO = DUO_;
     static constexpr int L = L_;
     static constexpr bool PAIR = PAIR_;
     static constexpr int MAXT = MAXT_;
@@ -36,7 +36,18 @@ struct Shape {
 // lanes, paired or not; a streamed tile at those and at one lane.  Anything
 // else returns `bad`.
 template <class R, class F>
-static R dispatch(int lanes, int pair, int deep, int stream, R bad, F&& f) {
+static R dispatch(int lanes, int pair, int deep, int stream, int duo, R bad, F&& f) {
+    if (duo) {
+        if (!hasDuo(lanes, pair) || (stream && lanes > 4)) return bad;
+        constexpr int B = kDeepThreads;
+        switch (lanes) {
+            case 1: return stream ? f(Shape<1, true, B, true, true>{}) : f(Shape<1, true, B, false, true>{});
+            case 2: return stream ? f(Shape<2, true, B, true, true>{}) : f(Shape<2, true, B, false, true>{});
+            case 4: return stream ? f(Shape<4, true, B, true, true>{}) : f(Shape<4, true, B, false, true>{});
+            case 8: return f(Shape<8, false, B, false, true>{});
+            default: return f(Shape<16, false, B, false, true>{});
+        }
+    }
     if (stream) {
         if (!hasStream(lanes, deep)) return bad;
         if (lanes == 1) return pair ? f(Shape<1, true, maxStepThreads(1), true>{}) : f(Shape<1, false, maxStepThreads(1), true>{});
@@ -68,13 +79,13 @@ static R dispatch(int lanes, int pair, int deep, int stream, R bad, F&& f) {
 
 template <class S>
 static auto kernelOf() {
-    return propagateKernel<S::L, PHOP_T, (bool)PHOP_SG, S::PAIR, S::MAXT, S::STREAM>;
+    return propagateKernel<S::L, PHOP_T, (bool)PHOP_SG, S::PAIR, S::MAXT, S::STREAM, S::DUO>;
 }
 
 cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t paramsBytes, int lanes, int ctas,
                                                     int threads, int smem, cudaStream_t stream) {
     if (paramsBytes != sizeof(StepParams)) return cudaErrorInvalidValue;  // objects built from different headers
-    return dispatch(lanes, p.pairSh, p.deepRegs, p.streamTile, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
+    return dispatch(lanes, p.pairSh, p.deepRegs, p.streamTile, p.duo, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
         auto k = kernelOf<decltype(shape)>();
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -85,8 +96,8 @@ cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t 
     });
 }
 
-int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int threads, int smem) {
-    return dispatch(lanes, pair, deep, stream, 0, [&](auto shape) -> int {
+int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, int threads, int smem) {
+    return dispatch(lanes, pair, deep, stream, duo, 0, [&](auto shape) -> int {
         auto k = kernelOf<decltype(shape)>();
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int n = 0;
@@ -95,8 +106,8 @@ int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream,
     });
 }
 
-cudaError_t PHOP_CAT(attributes_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, cudaFuncAttributes* a) {
-    return dispatch(lanes, pair, deep, stream, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
+cudaError_t PHOP_CAT(attributes_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, cudaFuncAttributes* a) {
+    return dispatch(lanes, pair, deep, stream, duo, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
         return cudaFuncGetAttributes(a, kernelOf<decltype(shape)>());
     });
 }

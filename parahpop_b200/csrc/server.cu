@@ -32,7 +32,8 @@ Server::Server(Engine& engine, const RunOptions& opt, int64_t capacity, double s
     lanes_ = opt.lanes > 0 ? opt.lanes : 2;
     // and one thread bound: the deep one at the server's own lane count, whose
     // slices are short of warps rather than of registers (40 requests of 1 to
-    // 3,000 objects: 124 -> 107 ms)
+    // 3,000 objects: 124 -> 107 ms; with the drag model on second warps 100
+    // -> 70)
     if (opt.lanes <= 0 && opt.deepRegs < 0) opt_.deepRegs = 1;
     PHOP_SCUDA(cudaSetDevice(engine.device()));
     PHOP_SCUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
@@ -300,7 +301,11 @@ int Server::step() {
         p.workCounter = ctl_;
         p.errorFlag = ctl_ + 1;
         PHOP_SCUDA(cudaEventRecord(ev0_, stream_));
-        engine_.launchStep(p, lanes_, opt_, false, stream_);
+        // a slice of one wave runs its drag model on second warps (the same
+        // results bit for bit)
+        RunOptions o = opt_;
+        o.duo = o.deepRegs > 0 && engine_.duoFits(nAct, lanes_);
+        engine_.launchStep(p, lanes_, o, false, stream_);
         PHOP_SCUDA(cudaEventRecord(ev1_, stream_));
         PHOP_SCUDA(cudaEventSynchronize(ev1_));
         launches += 1;
