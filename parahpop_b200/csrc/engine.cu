@@ -1516,8 +1516,8 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     // stage accelerations of its objects
     // warps in pairs: half of a CTA's warps hold objects; the static mail of
     // the pairs takes some shared memory
-    p.duo = opt.duo && hasDuo(L, p.pairSh) && (opt.threads <= 0 || opt.threads >= 64) && denv_.hasNrl && (denv_.bodyFlags[denv_.earthIndex] & kAtmosphere)
-            && p.splitRadius == 0.0;
+    p.nrl = nrlDrag();
+    p.duo = opt.duo && hasDuo(L, p.pairSh) && p.nrl && (opt.threads <= 0 || opt.threads >= 64) && p.splitRadius == 0.0;
     const int halves = p.duo ? 2 : 1;
     const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - (p.duo ? 4096 : 0) - bytes) / kStageBytes * L / 32 * 32 * halves; };
     const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
@@ -1539,11 +1539,11 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
         // never more threads than the compiled instantiation accepts (its
         // register count times the threads must fit the SM's register file)
         const int akey = ((((L * 2 + (opt.split ? 1 : 0)) * 2 + (shared ? 1 : 0)) * 2 + p.pairSh) * 2 + p.deepRegs) * 2
-                         + p.streamTile + 4096 * p.duo;
+                         + p.streamTile + 4096 * p.duo + 8192 * p.nrl;
         auto at = attrs_.find(akey);
         if (at == attrs_.end()) {
             cudaFuncAttributes a{};
-            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, p.duo, &a));
+            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, p.duo, p.nrl, &a));
             at = attrs_.emplace(akey, std::make_pair(a.maxThreadsPerBlock, a.numRegs)).first;
         }
         threadsReq = std::max(32 * halves, std::min(threadsReq, at->second.first / (32 * halves) * (32 * halves)));
@@ -1559,7 +1559,7 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
         if (it == occupancy_.end())
             it = occupancy_
                      .emplace(key, propagateMaxCtasPerSm(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, p.duo,
-                                                    threads, smem))
+                                                    p.nrl, threads, smem))
                      .first;
         perSm = it->second;
     }

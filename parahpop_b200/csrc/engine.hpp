@@ -242,17 +242,21 @@ private:
     // stride `stride`); `slots` (nullable) lists the objects to order
     const int64_t* orderByRadius(int64_t n, const double* dState, cudaStream_t stream, int64_t* launches,
                                  int64_t stride = 0, const int64_t* slots = nullptr);
+    // Whether the Earth's drag model is NRLMSISE-00.
+    bool nrlDrag() const {
+        return denv_.hasNrl && denv_.earthIndex >= 0 && (denv_.bodyFlags[denv_.earthIndex] & kAtmosphere) != 0;
+    }
     // Whether a batch is small enough for the drag model on a second warp:
     // one wave of main warps (four of a CTA's eight).  Beyond it the idle
     // partners of objects above the atmosphere and the halved main warps cost
     // more than the overlap gives (10^4 LEO objects at four lanes, 2.1 waves:
     // 7.6 -> 11.4 ms a twelve-step probe; 4,000 objects, one wave: 4.8 -> 3.3).
     bool duoFits(int64_t n, int lanes) const {
-        return denv_.hasNrl && (n * lanes + 31) / 32 <= (int64_t)sms_ * (kDeepThreads / 64);
+        return nrlDrag() && (n * lanes + 31) / 32 <= (int64_t)sms_ * (kDeepThreads / 64);
     }
     // The order only keeps warps together in the NRLMSISE-00 branches: without
     // that model the sort (a key kernel and six of CUB's) would buy nothing.
-    bool ordersObjects(const RunOptions& opt) const { return opt.ordered && denv_.hasNrl; }
+    bool ordersObjects(const RunOptions& opt) const { return opt.ordered && nrlDrag(); }
     void buildRecordGrid(double lo, double hi, TimeGrid& g, cudaStream_t stream, int64_t* launches);
     LaunchShape launchStep(StepParams p, int lanes, const RunOptions& opt, bool shared, cudaStream_t stream);
     LaunchShape prepareStep(StepParams& p, int lanes, const RunOptions& opt, bool shared);

@@ -230,8 +230,9 @@ template <> struct PairRows<float> {
 };
 // `pairs` row pairs of a column from its first 16-byte chunk.  kShared: a staged tile is
 // read by shared-memory loads, in a loop of its own, two row pairs an
-// iteration (four in FP32: one CTA of eight warps, one lane per object, 82.7
-// against 85.7 thousand cycles an evaluation at degree 70).  Such a load whose lanes differ in at most two addresses (W <=
+// iteration (four measured better in FP32 by itself, 82.7 against 85.7
+// thousand cycles an evaluation at degree 70, but worse in the whole kernel,
+// whose instructions it crowds: 10^6 uneven objects 109 against 103 ms).  Such a load whose lanes differ in at most two addresses (W <=
 // 2) takes 2 cycles of an SM per 16 bytes of a warp, a generic load 4, and
 // the column loop of one lane per object was bound by the latter (82 % of the
 // load path's peak, FP64 pipe 52 %): 200,000 uneven objects x 8 steps FP64
@@ -250,7 +251,7 @@ static __device__ __forceinline__ void fieldRows(const TileRef& tile, TileStream
     constexpr int kChunks = PairRows<T>::kChunks, kStep = kChunks * W;
     if (MODE == TileRead::kShared && tile.staged) {
         const Chunk* tp = (const Chunk*)g_smem + chunk + pj;
-#pragma unroll(sizeof(T) == 8 ? 2 : 4)
+#pragma unroll 2
         for (int i = 0; i < pairs; ++i, tp += kStep) {
             PairRows<T> r;
             r.template load<W>(tp);

@@ -186,6 +186,7 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.state = dState;
     sp.bc = dBc;
     sp.ams = dAms;
+    sp.nrl = nrlDrag();
     sp.nsteps = K;
     sp.stepT0 = dT0;
     sp.stepDt = dDt;
@@ -203,7 +204,7 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.useSmemTile = opt.tileSmem != 0 && tileBytes + 1024 <= maxSmem_ && fit(tileBytes) >= 64;
     const int threads = std::min(threadsReq, fit(sp.useSmemTile ? tileBytes : 0));
     const int smem = propagateSmemBytes(sp, L, threads);
-    int perSm = opt.ctasPerSm > 0 ? opt.ctasPerSm : propagateMaxCtasPerSm(L, opt.split, true, 0, 0, 0, 0, threads, smem);
+    int perSm = opt.ctasPerSm > 0 ? opt.ctasPerSm : propagateMaxCtasPerSm(L, opt.split, true, 0, 0, 0, 0, sp.nrl, threads, smem);
     if (perSm <= 0) perSm = 1;
     const int64_t groups = (n + (32 / L) - 1) / (32 / L);
     const int64_t need = (groups + threads / 32 - 1) / (threads / 32);

@@ -10,8 +10,8 @@ namespace phop {
 #define PHOP_DECL(sfx)                                                                                     \
     cudaError_t launchPropagate_##sfx(const StepParams& p, size_t paramsBytes, int lanes, int ctas, int threads, \
                                       int smem, cudaStream_t stream);                                       \
-    int occupancy_##sfx(int lanes, int pair, int deep, int stream, int duo, int threads, int smem);                \
-    cudaError_t attributes_##sfx(int lanes, int pair, int deep, int stream, int duo, cudaFuncAttributes* a);
+    int occupancy_##sfx(int lanes, int pair, int deep, int stream, int duo, int nrl, int threads, int smem);                \
+    cudaError_t attributes_##sfx(int lanes, int pair, int deep, int stream, int duo, int nrl, cudaFuncAttributes* a);
 PHOP_DECL(f64_grid)
 PHOP_DECL(f64_mixed)
 PHOP_DECL(f32_grid)
@@ -98,17 +98,17 @@ int propagateSmemBytes(const StepParams& p, int lanes, int threads) {
     return (p.useSmemTile ? p.tileBytes : p.streamTile ? threads / (p.duo ? 64 : 32) * kRingBytes : 0) + kStageBytes * (threads / (p.duo ? 2 : 1) / lanes);
 }
 
-int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int threads, int smem) {
+int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, int threads, int smem) {
     if (split)
-        return shared ? occupancy_f32_grid(lanes, pair, deep, stream, duo, threads, smem)
-                      : occupancy_f32_mixed(lanes, pair, deep, stream, duo, threads, smem);
-    return shared ? occupancy_f64_grid(lanes, pair, deep, stream, duo, threads, smem)
-                  : occupancy_f64_mixed(lanes, pair, deep, stream, duo, threads, smem);
+        return shared ? occupancy_f32_grid(lanes, pair, deep, stream, duo, nrl, threads, smem)
+                      : occupancy_f32_mixed(lanes, pair, deep, stream, duo, nrl, threads, smem);
+    return shared ? occupancy_f64_grid(lanes, pair, deep, stream, duo, nrl, threads, smem)
+                  : occupancy_f64_mixed(lanes, pair, deep, stream, duo, nrl, threads, smem);
 }
 
-cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, cudaFuncAttributes* a) {
-    if (split) return shared ? attributes_f32_grid(lanes, pair, deep, stream, duo, a) : attributes_f32_mixed(lanes, pair, deep, stream, duo, a);
-    return shared ? attributes_f64_grid(lanes, pair, deep, stream, duo, a) : attributes_f64_mixed(lanes, pair, deep, stream, duo, a);
+cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, cudaFuncAttributes* a) {
+    if (split) return shared ? attributes_f32_grid(lanes, pair, deep, stream, duo, nrl, a) : attributes_f32_mixed(lanes, pair, deep, stream, duo, nrl, a);
+    return shared ? attributes_f64_grid(lanes, pair, deep, stream, duo, nrl, a) : attributes_f64_mixed(lanes, pair, deep, stream, duo, nrl, a);
 }
 
 cudaError_t launchPropagate(const StepParams& p, int lanes, bool split, bool shared, int ctas, int threads,

@@ -95,6 +95,7 @@ struct StepParams {
     int streamTile;         // the tile streamed through rings in shared memory (hasStream shapes)
     int pairSh;             // the geopotential of lane-group pairs (tile built for 2L lanes)
     int duo;                // warps in pairs, the drag model on the second (hasDuo shapes)
+    int nrl;                // the kernel with NRLMSISE-00 (a configuration that uses it needs it)
     int deepRegs;           // host-side choice of the kernel's thread bound (stepThreadBound)
     int tileWaitTest;       // test of the staging time-out: arm the barrier, issue no copy
     // scheduling and errors
@@ -135,10 +136,10 @@ void launchRecordPairs(const EpochRecord* grid, int64_t count, double2* pairs, c
 cudaError_t launchPropagate(const StepParams& p, int lanes, bool split, bool shared, int ctas, int threads,
                             cudaStream_t stream);
 int propagateSmemBytes(const StepParams& p, int lanes, int threads);
-int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int threads, int smem);
+int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, int threads, int smem);
 // The compiled instantiation's attributes (maxThreadsPerBlock, numRegs,
 // localSizeBytes): the launch shape never asks for more threads than the
 // instantiation accepts.
-cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, cudaFuncAttributes* a);
+cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, cudaFuncAttributes* a);
 
 }  // namespace phop

@@ -23,9 +23,11 @@ namespace phop {
 
 // one compiled step-kernel shape: lanes per object, lane-group pairs, thread
 // bound, the tile streamed through rings, the drag model on a second warp
-template <int L_, bool PAIR_, int MAXT_, bool STREAM_ = false, bool DUO_ = false>
+template <int L_, bool PAIR_, int MAXT_, bool STREAM_ = false, bool DUO_ = false, bool NRL_ = true>
 struct Shape {
-    static constexpr bool STREAM = STREAM_, DUO = DUO_;
+    static constexpr bool STREAM = STREAM_, DUO = DUO_, NRL = NRL_;
+    // the same shape without NRLMSISE-00
+    using Bare = Shape<L_, PAIR_, MAXT_, STREAM_, DUO_, false>;
     static constexpr int L = L_;
     static constexpr bool PAIR = PAIR_;
     static constexpr int MAXT = MAXT_;
@@ -36,7 +38,7 @@ struct Shape {
 // lanes, paired or not; a streamed tile at those and at one lane.  Anything
 // else returns `bad`.
 template <class R, class F>
-static R dispatch(int lanes, int pair, int deep, int stream, int duo, R bad, F&& f) {
+static R dispatchShape(int lanes, int pair, int deep, int stream, int duo, R bad, F&& f) {
     if (duo) {
         if (!hasDuo(lanes, pair) || (stream && lanes > 4)) return bad;
         constexpr int B = kDeepThreads;
@@ -77,15 +79,28 @@ static R dispatch(int lanes, int pair, int deep, int stream, int duo, R bad, F&&
     }
 }
 
+// with or without the NRLMSISE-00 model (duo shapes always have it)
+template <class R, class F>
+static R dispatch(int lanes, int pair, int deep, int stream, int duo, int nrl, R bad, F&& f) {
+    return dispatchShape(lanes, pair, deep, stream, duo, bad, [&](auto shape) -> R {
+        using S = decltype(shape);
+        if constexpr (S::DUO) {
+            return nrl ? f(S{}) : bad;
+        } else {
+            return nrl ? f(S{}) : f(typename S::Bare{});
+        }
+    });
+}
+
 template <class S>
 static auto kernelOf() {
-    return propagateKernel<S::L, PHOP_T, (bool)PHOP_SG, S::PAIR, S::MAXT, S::STREAM, S::DUO>;
+    return propagateKernel<S::L, PHOP_T, (bool)PHOP_SG, S::PAIR, S::MAXT, S::STREAM, S::NRL, S::DUO>;
 }
 
 cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t paramsBytes, int lanes, int ctas,
                                                     int threads, int smem, cudaStream_t stream) {
     if (paramsBytes != sizeof(StepParams)) return cudaErrorInvalidValue;  // objects built from different headers
-    return dispatch(lanes, p.pairSh, p.deepRegs, p.streamTile, p.duo, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
+    return dispatch(lanes, p.pairSh, p.deepRegs, p.streamTile, p.duo, p.nrl, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
         auto k = kernelOf<decltype(shape)>();
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -96,8 +111,8 @@ cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t 
     });
 }
 
-int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, int threads, int smem) {
-    return dispatch(lanes, pair, deep, stream, duo, 0, [&](auto shape) -> int {
+int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, int nrl, int threads, int smem) {
+    return dispatch(lanes, pair, deep, stream, duo, nrl, 0, [&](auto shape) -> int {
         auto k = kernelOf<decltype(shape)>();
         if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int n = 0;
@@ -106,8 +121,8 @@ int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream,
     });
 }
 
-cudaError_t PHOP_CAT(attributes_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, cudaFuncAttributes* a) {
-    return dispatch(lanes, pair, deep, stream, duo, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
+cudaError_t PHOP_CAT(attributes_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, int nrl, cudaFuncAttributes* a) {
+    return dispatch(lanes, pair, deep, stream, duo, nrl, cudaErrorInvalidValue, [&](auto shape) -> cudaError_t {
         return cudaFuncGetAttributes(a, kernelOf<decltype(shape)>());
     });
 }
