@@ -141,7 +141,7 @@ int phop_propagate_trajectory(phop_context* ctx, int64_t n, double epoch_mjd2000
  * has reserved the GPU's memory, a real-time loop that cannot take the
  * device-wide synchronisation a cudaMalloc or cudaFree may imply, or a
  * service that fixes its memory footprint at start-up.  Scratch comes from
- * one 4 MiB device array built into the library, held on every GPU that
+ * one 5 MiB device array built into the library, held on every GPU that
  * loads it until the process exits; the call allocates nothing.  The caller
  * passes device arrays: d_states_soa (6*n doubles, updated in place), d_bc =
  * cd * area / mass and d_ams = cr_eff * area / mass (area in km^2, cr_eff =
@@ -179,7 +179,8 @@ int phop_propagate_device_noalloc(phop_context* ctx, int64_t n, double* d_states
  *              launch parameters (replayed for repeated batches), 0 = plain
  *              launches
  *   "tile_smem"  1 (default) = stage the coefficient tile in shared memory
- *              when it fits, 0 = read it through L1 (more threads per SM)
+ *              when it fits, or stream it through rings there (one lane per
+ *              object, and the deep thread bound); 0 = read it through L1
  *   "pair_sh"  geopotential of lane-group pairs, two objects per lane
  *              (each coefficient loaded from shared memory serves both;
  *              packed FP32 in split precision; at one, two or four lanes

@@ -17,8 +17,9 @@
 //
 // Limits: at most kMaxSteps (256) fixed steps per call and a coefficient tile
 // of at most 512 KiB at one entry per term (withinTileLimit; enough for
-// degree/order 120 in FP64); calls beyond them are rejected with an error.  Every GPU that loads the library
-// holds the array (4 MiB) until the process exits.  All calls share it: the
+// degree/order 120 in FP64); calls beyond them are rejected with an error.
+// Every GPU that loads the library holds the array (5 MiB) until the process
+// exits.  All calls share it: the
 // control words are cleared on every call, the tile is re-copied whenever a
 // call needs another one than the array holds (keyed by the context's
 // never-reused serial number, the lane count and the precision), and calls
@@ -40,10 +41,10 @@
 
 namespace phop {
 
-constexpr size_t kStaticScratchBytes = 4u << 20;
+constexpr size_t kStaticScratchBytes = 5u << 20;
 constexpr int kMaxSteps = 256;
 constexpr size_t kCtlBytes = 256;
-constexpr size_t kTileBytes = 640u << 10;
+constexpr size_t kTileBytes = 1216u << 10;
 
 static __device__ __align__(256) unsigned char g_staticScratch[kStaticScratchBytes];
 
@@ -74,8 +75,10 @@ const HostTile& Engine::hostTileFor(int L, bool split, int lowDeg) {
 // The entry point's size limit, stated for a tile of one 48-byte (FP64) or
 // 32-byte (split precision) entry per term above degree `lowDeg`, columns in
 // blocks of L padded to the block's longest, and 8 bytes per block.  The
-// tile in use holds more bytes per term; kTileBytes is what the largest
-// field within the limit needs (629,904 bytes, degree 145 at four lanes).
+// tile in use holds more bytes per term and whole row pairs of every column;
+// kTileBytes is what the largest field within the limit needs (1,230,848
+// bytes, degree 1373 and order 7 at eight lanes, FP64; of fields of all
+// orders 629,904 bytes before the padding, degree 145 at four lanes).
 static bool withinTileLimit(int N, int M, int L, bool split, int lowDeg) {
     const int nb = (M + L) / L;
     int64_t entries = 0;
