@@ -40,27 +40,28 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT))
 
 METRIC = "object-steps/s full-force at ≤1 cm vs FP64 oracle; p50/p99 request latency"
-SH_FLOP_PER_TERM = 29  # algorithmic FLOPs per (n, m) term of the SH recursion
+SH_FLOP_PER_TERM = 18  # algorithmic FLOPs per row of the field's column sums: a recurrence step and six sums
+SH_EVALUATIONS = 12.0  # force evaluations per step (the thirteenth stage serves only the error estimate)
 SPLIT_TOL_M = 1e-2
 FP64_TOL_M = 1e-3
 
 
 def sh_terms(degree: int) -> float:
-    return (degree + 1) * (degree + 2) / 2.0
+    return (degree + 2) * (degree + 3) / 2.0
 
 
 def sh_flops_per_object_step(degree: int) -> float:
-    return 13.0 * SH_FLOP_PER_TERM * sh_terms(degree)
+    return SH_EVALUATIONS * SH_FLOP_PER_TERM * sh_terms(degree)
 
 
 # DRAM bytes (read + write) per object-step of the step kernel, from ncu
 # captures (profiles/): the state is read once and written once per launch
 # (~100 B per object); the rest is local memory written back from L2 and the
-# epoch-record grid.  c3: the split form's kernel at two lanes with lane-group
-# pairs and the 256-thread bound, 10^5 objects x 24 steps (8.77 + 5.82 GB over
-# 2,391,620 object-steps); the other workloads have no capture of the current
-# kernel (null).
-NCU_BYTES_PER_OBJECT_STEP = {"c3": (8.769621e9 + 5.815049e9) / 2_391_620, "c1": None, "c2": None}
+# epoch-record grid.  c3: the split form's kernel at one lane with lane-group
+# pairs, 10^5 objects x 24 steps (17.09 + 6.43 GB over 2,391,620
+# object-steps); the other workloads have no capture of the current kernel
+# (null).
+NCU_BYTES_PER_OBJECT_STEP = {"c3": (17.090873e9 + 6.427766e9) / 2_391_620, "c1": None, "c2": None}
 
 
 def dist_env():
@@ -622,7 +623,7 @@ def main():
         achieved = flops / (r["kernel_ms"] * 1e-3) * 1e-12
         if head == "split":
             low = args.split_degree or (24 if degree > 80 else 20)  # the library's default by field degree
-            f64 = 13.0 * SH_FLOP_PER_TERM * sh_terms(low)
+            f64 = SH_EVALUATIONS * SH_FLOP_PER_TERM * sh_terms(low)
             f32 = sh_flops_per_object_step(degree) - f64
             peak = sh_flops_per_object_step(degree) / (f64 / fp64_peak + f32 / fp32_peak)
             peak_note = (f"FMA peaks measured on this GPU (phop_fma_peak: FP64 {fp64_peak:.1f}, FP32 "
@@ -650,12 +651,12 @@ def main():
             "roofline": {"bound": "fp64+fp32" if head == "split" else "fp64", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak if peak > 0 else None,
                          "traffic": per_os * steps_per_launch if per_os else None,
-                         "traffic_note": "DRAM read+write bytes per launch: ncu capture of the split kernel at two "
-                                         "lanes, lane-group pairs, 256-thread bound (6.1 KB per object-step: "
+                         "traffic_note": "DRAM read+write bytes per launch: ncu capture of the split kernel at one "
+                                         "lane, lane-group pairs, 256-thread bound (9.8 KB per object-step: "
                                          "local-memory write-back and epoch-record reads) times the object-steps of "
                                          "one timed launch" if per_os else None,
                          "peak_source": peak_note,
-                         "numerator": f"29 FLOP x (N+1)(N+2)/2 SH terms x 13 stages per object-step, N = {degree}"},
+                         "numerator": f"18 FLOP x (N+2)(N+3)/2 rows x 12 evaluations per object-step, N = {degree}"},
             "cpu_baseline": cpu,
             "reference_gpu": ref_gpu,
             "e2e": {"value": h["e2e_value"], "unit": "object-steps/s", "h2d_bytes_per_step": r["e2e"]["h2d_bytes"],

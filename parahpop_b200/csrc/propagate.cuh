@@ -1,7 +1,7 @@
 // Fused batched RKF78 propagation kernels for sm_100a.
 //
 // One persistent kernel advances object groups through all their fixed steps:
-// the 13 RKF78 stages, the full force model and the 8th-order update run on
+// the RKF78 stages, the full force model and the 8th-order update run on
 // chip (registers and shared memory), so the only per-object HBM traffic is the
 // state read at the start and written at the end of the whole propagation.
 //
