@@ -1478,10 +1478,10 @@ void Engine::launchStepGraph(const StepParams& p, const LaunchShape& shape, cons
 }
 
 // FP64 low part of each column in split precision (the FP64 form ignores
-// it): n <= the option's degree.  Its default follows the field's degree: the
-// FP32 rounding of the recursion accumulates over more terms in a larger
-// field (24 h, 10^5 LEO objects at degree 120: 11.5 mm max with n <= 20 in
-// FP64, 8.3 mm with n <= 24; degree 70: 6.4 mm with n <= 20).
+// it): n <= the option's degree, and the margin beyond it (geopotential.hpp).
+// Its default follows the field's degree: the FP32 rounding of the recursion
+// accumulates over more terms in a larger field (24 h: 5.3 mm max for 10^4
+// LEO objects at degree 70 with 20, 8.0 mm for 10^5 at degree 120 with 24).
 int lowDegreeFor(const RunOptions& opt, int fieldDegree) {
     if (!opt.split) return kLowDeg;
     const int d = opt.splitFp64Degree > 0 ? opt.splitFp64Degree

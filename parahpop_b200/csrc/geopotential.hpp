@@ -27,15 +27,26 @@
 // ((i chunks + c) W + j): the lanes of a load read consecutive 16-byte words,
 // and a block's pairs follow the block's before: the tile is one stream in
 // the order the column loop reads it.  In split precision a block's FP64
-// pairs come first, then its FP32 pairs; the rows of degrees n <= lowDeg + 1
-// of a column are FP64, rounded up to whole pairs (by the column alone: the
-// same rows whatever W).  The one degree more than asked for costs 1.6 % of
-// the rows at degree 70 and keeps the FP32 error below that of the
-// spherical-component sums this form replaced (20,000 LEO objects, 30 steps
-// of 60 s, rms against FP64 at degrees 36 / 70 / 90 / 120: 0.81 / 1.20 / 0.94
-// / 0.96 um; those sums 0.89 / 1.26 / 0.98 / 1.02 um; without the degree 0.90
-// / 1.30 / 1.03 / 1.03 um).  The bytes are padded to whole stages of the
-// stream (kStageChunks).
+// pairs come first, then its FP32 pairs; the rows of degrees n <= lowDeg +
+// kLowMargin of a column are FP64, rounded up to whole pairs (by the column
+// alone: the same rows whatever W).  The bytes are padded to whole stages of
+// the stream (kStageChunks).
+//
+// kLowMargin: in this form the FP32 rounding of the row factors A is the same
+// field error in every evaluation, and that of alpha sin phi and alpha^2 the
+// same in every row of one, so the error of a day's orbit comes out larger
+// than that of the spherical-component sums this form replaced although the
+// error of one evaluation does not.  Split against FP64 after 24 h, mm, p99 /
+// max, at low parts of 20 (degree 70) and 24 (degree 120): 10^4 LEO objects
+// at degree 70, 10^5 of the uneven population, 10^5 LEO at degree 120
+//     spherical components   1.93 / 6.41   0.74 / 6.31   1.64 / 8.29
+//     margin 1               2.49 / 9.45   0.97 / 9.45   1.91 / 11.64
+//     margin 9               1.37 / 6.08   0.55 / 5.57   1.15 / 6.97
+//     margin 11              1.27 / 5.30   0.51 / 5.67   1.01 / 7.99
+// The ten FP64 degrees beyond the first cost 7 % of the first run's time, 4 %
+// of the second's and 6 % of the third's (nine FP64 degrees the same).  Two
+// words for alpha sin phi and alpha^2 instead took 5, 11 and 11 % and left
+// 1.80 / 6.94, 0.81 / 9.24 and 1.46 / 6.96.
 #pragma once
 #include <vector>
 
@@ -50,16 +61,20 @@ namespace phop {
 constexpr int kChunks64 = 7;  // 16-byte chunks of an FP64 row pair
 constexpr int kChunks32 = 4;  // and of an FP32 row pair
 
-// FP64 row pairs of column M in a field of degree N whose FP64 low part is
-// `lowDeg` (lowDeg >= N: all rows); they fall with M
+constexpr int kLowMargin = 11;  // FP64 degrees beyond lowDeg: see above
+
+// row nu of the last FP64 degree in a field of degree N whose FP64 low part
+// is `lowDeg`
+PHOP_GEO_HD int topRow64(int N, int lowDeg) { return (lowDeg + kLowMargin < N ? lowDeg + kLowMargin : N) + 1; }
+// FP64 row pairs of column M (lowDeg >= N: all rows); they fall with M
 PHOP_GEO_HD int rowPairs64(int M, int N, int lowDeg) {
-    const int top = lowDeg + 1 < N ? lowDeg + 2 : N + 1;
+    const int top = topRow64(N, lowDeg);
     const int rows = top - M + 1;
     return rows > 0 ? (rows + 1) / 2 : 0;
 }
 // FP32 row pairs that hold those of every column >= M
 PHOP_GEO_HD int rowPairs32(int M, int N, int lowDeg) {
-    const int top = lowDeg + 1 < N ? lowDeg + 2 : N + 1;
+    const int top = topRow64(N, lowDeg);
     const int rows = N + 1 - (M <= top ? top : M - 1);
     return rows > 0 ? (rows + 1) / 2 : 0;
 }

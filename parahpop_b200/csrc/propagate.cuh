@@ -39,8 +39,8 @@
 namespace phop {
 
 // Split precision keeps degrees n <= splitFp64Degree (by default 20, or 24
-// for fields above degree 80; at most kLowMax) of every column in FP64 and
-// runs the rest in FP32.
+// for fields above degree 80; at most kLowMax) of every column in FP64, with
+// a margin beyond (geopotential.hpp), and runs the rest in FP32.
 constexpr int kLowDeg = 8;                                  // smallest FP64 low part of the split form
 constexpr int kSplitFp64Degree = 20;                        // split form default up to degree 80
 constexpr int kSplitFp64DegreeHigh = 24;                    // split form default above degree 80
