@@ -470,8 +470,18 @@ struct Duo {
     int* quit;
     int barrier;    // the post barrier; the reply barrier is the next
 };
-static __device__ __forceinline__ void duoArrive(int id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
-static __device__ __forceinline__ void duoSync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+// Both forms are aligned: all lanes of a warp execute them together, which the
+// force model's per-lane branches (shadow, spheres of influence) before the
+// reply would otherwise leave to the compiler.  The warp's synchronisation
+// also orders its lanes' accesses to the mail.
+static __device__ __forceinline__ void duoArrive(int id) {
+    __syncwarp();
+    asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory");
+}
+static __device__ __forceinline__ void duoSync(int id) {
+    __syncwarp();
+    asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+}
 
 // the partner's loop
 template <int L>
@@ -484,7 +494,6 @@ static __device__ __forceinline__ void duoPartner(const DevEnv& e, const Duo& du
         const double f[3] = {m.f[0], m.f[1], m.f[2]};
         const double rho = nrlDensity<L>(e, NrlTime{m.sec, m.gast, m.block, m.valid}, f);
         if (lane % L == 0) m.rho = rho;
-        __syncwarp();
         duoArrive(duo.barrier + 1);
     }
 }
@@ -513,7 +522,6 @@ static __device__ __forceinline__ void accelerations(const StepParams& p, const 
             m.block = t.block;
             m.valid = t.valid;
         }
-        __syncwarp();
         duoArrive(duo.barrier);
     }
     for (int bi = 0; bi < e.nbodies; ++bi) {
@@ -993,7 +1001,6 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
     }
     if constexpr (DUO) {
         if ((threadIdx.x & 31) == 0) *duo.quit = 1;
-        __syncwarp();
         duoArrive(duo.barrier);
     }
     if constexpr (STREAM) stream.end();
