@@ -1512,44 +1512,36 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
         p.nblocks64 = full.nblocks;
         p.splitRadius = host_.shR + opt.splitFloorKm;
     }
-    // shared memory per CTA: the coefficient tile (when it fits) plus the
-    // stage accelerations of its objects
-    // warps in pairs: half of a CTA's warps hold objects; the static mail of
-    // the pairs takes some shared memory
+    // warps in pairs: half of a CTA's warps hold objects
     p.nrl = nrlDrag();
     p.duo = opt.duo && hasDuo(L, p.pairSh) && p.nrl && (opt.threads <= 0 || opt.threads >= 64) && p.splitRadius == 0.0;
     const int halves = p.duo ? 2 : 1;
-    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - (p.duo ? 4096 : 0) - bytes) / kStageBytes * L / 32 * 32 * halves; };
-    const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
-                      * (32 * halves);
-    const int staged = opt.tileSmem != 0 && tile.bytes + 1024 <= maxSmem_ ? fit(tile.bytes) : 0;
-    p.useSmemTile = staged >= 64;
-    // A tile that does not fit, or leaves room for fewer than three quarters
-    // of the threads, is streamed through a ring per warp where the kernel
-    // can (a streamed row costs about a fifth more than a staged one);
-    // "tile_smem" = 0 asks for reads through L1, and the FP64 floor of the
-    // split form lets a warp's objects part in the row loop.
-    const int streamed = (maxSmem_ - 1024 - (p.duo ? 4096 : 0)) / (kRingBytes + kStageBytes * (32 / L)) * 32 * halves;
-    p.streamTile = opt.tileSmem != 0 && (p.duo ? L <= 4 : hasStream(L, p.deepRegs)) && tile.nblocks > 0 && p.splitRadius == 0.0
-                   && std::min(staged, bound) < std::min(streamed, bound) * 3 / 4;
-    if (p.streamTile) p.useSmemTile = 0;
-    int registers = 0;
-    int threadsReq = bound;
-    {
-        // never more threads than the compiled instantiation accepts (its
-        // register count times the threads must fit the SM's register file)
-        const int akey = ((((L * 2 + (opt.split ? 1 : 0)) * 2 + (shared ? 1 : 0)) * 2 + p.pairSh) * 2 + p.deepRegs) * 2
-                         + p.streamTile + 4096 * p.duo + 8192 * p.nrl;
-        auto at = attrs_.find(akey);
+    const auto attributes = [&](int stream) -> const KernelAttributes& {
+        const int key = ((((L * 2 + (opt.split ? 1 : 0)) * 2 + (shared ? 1 : 0)) * 2 + p.pairSh) * 2 + p.deepRegs) * 2
+                        + stream + 4096 * p.duo + 8192 * p.nrl;
+        auto at = attrs_.find(key);
         if (at == attrs_.end()) {
             cudaFuncAttributes a{};
-            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, p.streamTile, p.duo, p.nrl, &a));
-            at = attrs_.emplace(akey, std::make_pair(a.maxThreadsPerBlock, a.numRegs)).first;
+            PHOP_CUDA(propagateAttributes(L, opt.split, shared, p.pairSh, p.deepRegs, stream, p.duo, p.nrl, &a));
+            at = attrs_.emplace(key, KernelAttributes{a.maxThreadsPerBlock, a.numRegs, (int)a.sharedSizeBytes}).first;
         }
-        threadsReq = std::max(32 * halves, std::min(threadsReq, at->second.first / (32 * halves) * (32 * halves)));
-        registers = at->second.second;
-    }
-    int threads = std::min(threadsReq, p.useSmemTile ? staged : p.streamTile ? streamed : fit(0));
+        return at->second;
+    };
+    // "tile_smem" = 0 asks for reads through L1, and the FP64 floor of the
+    // split form lets a warp's objects part in the row loop: no stream
+    const bool mayStream = opt.tileSmem != 0 && (p.duo ? L <= 4 : hasStream(L, p.deepRegs)) && tile.nblocks > 0
+                           && p.splitRadius == 0.0;
+    const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
+                      * (32 * halves);
+    const StepRoom room = stepRoom(maxSmem_, attributes(0).smem, mayStream ? attributes(1).smem : 0, tile.bytes, L,
+                                   p.duo != 0, bound, opt.tileSmem != 0, mayStream);
+    p.useSmemTile = room.staged;
+    p.streamTile = room.streamed;
+    // never more threads than the compiled instantiation accepts (its
+    // register count times the threads must fit the SM's register file)
+    const KernelAttributes& own = attributes(p.streamTile);
+    const int registers = own.registers;
+    int threads = std::min(std::max(32 * halves, std::min(bound, own.threads / (32 * halves) * (32 * halves))), room.threads);
     int perSm = opt.ctasPerSm;
     if (perSm <= 0) {
         const int smem = propagateSmemBytes(p, L, threads);
@@ -1563,6 +1555,7 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
                      .first;
         perSm = it->second;
     }
+    const bool fits = perSm > 0;
     if (perSm <= 0) perSm = 1;
     // one warp per group of 32 / L objects; when every group fits one wave,
     // spread the warps evenly over all SMs instead of filling CTAs first
@@ -1580,6 +1573,7 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     shape.ctas = (int)std::max<int64_t>(1, std::min<int64_t>(slots, need));
     shape.smemTile = p.useSmemTile != 0;
     shape.registers = registers;
+    shape.fits = fits;
     return shape;
 }
 
@@ -1663,6 +1657,7 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
             }
             StepParams q = p;
             const LaunchShape shape = prepareStep(q, L, o, shared);
+            if (!shape.fits) break;
             PHOP_CUDA(cudaEventRecord(e0, stream));
             enqueueStep(q, shape, o, shared, stream);
             PHOP_CUDA(cudaEventRecord(e1, stream));

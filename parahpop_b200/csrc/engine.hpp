@@ -215,6 +215,7 @@ public:
         int lanes = 0, threads = 0, ctas = 0;
         int registers = 0;  // registers a thread of the chosen instantiation
         bool smemTile = false;
+        bool fits = true;  // whether a CTA of this shape fits an SM
     };
     // Per-batch time description handed to the step kernel.
     struct TimeGrid {
@@ -295,7 +296,10 @@ private:
     std::map<int, HostTile> hostTiles_;
     std::map<int, int> tuned_;  // autotuned lane count per batch class
     std::map<int64_t, int> occupancy_;  // resident CTAs per SM by launch configuration
-    std::map<int, std::pair<int, int>> attrs_;  // maxThreadsPerBlock, numRegs of each step-kernel instantiation
+    struct KernelAttributes {
+        int threads, registers, smem;  // maxThreadsPerBlock, numRegs, sharedSizeBytes
+    };
+    std::map<int, KernelAttributes> attrs_;  // of each step-kernel instantiation
 };
 
 }  // namespace phop

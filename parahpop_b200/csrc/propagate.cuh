@@ -35,6 +35,7 @@
 #include <stdint.h>
 
 #include "device_env.cuh"
+#include "geopotential.hpp"
 
 namespace phop {
 
@@ -130,16 +131,53 @@ __host__ __device__ constexpr int stepThreadBound(int lanes, int deep, int duo =
     return duo || (deep && hasDeepShape(lanes)) ? kDeepThreads : maxStepThreads(lanes);
 }
 
+// Shared memory of a step CTA: what a kernel holds by itself (the staging
+// barrier; a duo kernel's mail, 7,296 bytes at one lane), the staged tile or
+// the warps' rings, and the stage accelerations of the objects.  At least
+// 1 KiB beside the dynamic part is left to the kernel.
+constexpr int kDuoPairs = 4;  // warp pairs of a CTA of kDeepThreads threads
+struct DuoMail {
+    double f[3], sec, gast;
+    int block, valid;
+    double rho;
+};
+struct StepRoom {
+    int threads = 0;          // most threads the shared memory has room for
+    bool staged = false, streamed = false;
+};
+// A tile that does not fit, or leaves room for fewer than three quarters of
+// the threads, is streamed through a ring per warp where the kernel can (a
+// streamed row costs about a fifth more than a staged one).  maxSmem: what a
+// CTA may use in all; ownStaged, ownStreamed: what the kernels with and
+// without a stream hold by themselves; bound: the threads asked for.
+inline StepRoom stepRoom(int maxSmem, int ownStaged, int ownStreamed, int tileBytes, int lanes, bool duo, int bound,
+                         bool mayStage, bool mayStream) {
+    const int halves = duo ? 2 : 1;  // half of a duo CTA's warps hold objects
+    const auto room = [&](int own) { return maxSmem - (own > 1024 ? own : 1024); };
+    const auto fit = [&](int bytes) {
+        return bytes < room(ownStaged) ? (room(ownStaged) - bytes) / kStageBytes * lanes / 32 * 32 * halves : 0;
+    };
+    const int staged = mayStage ? fit(tileBytes) : 0;
+    const int streamed = mayStream ? room(ownStreamed) / (kRingBytes + kStageBytes * (32 / lanes)) * 32 * halves : 0;
+    const auto most = [&](int t) { return t < bound ? t : bound; };
+    StepRoom r;
+    r.streamed = mayStream && most(staged) < most(streamed) * 3 / 4;
+    r.staged = !r.streamed && staged >= 64;
+    r.threads = r.staged ? staged : r.streamed ? streamed : fit(0);
+    return r;
+}
+
 void launchEpochRecords(const DevEnv& env, const double* epochs, int count, EpochRecord* out, cudaStream_t stream);
 // pairs[(k * kInterpFields + f)] = {field f of grid[k], of grid[k + 1]}, k < count - 1
 void launchRecordPairs(const EpochRecord* grid, int64_t count, double2* pairs, cudaStream_t stream);
 cudaError_t launchPropagate(const StepParams& p, int lanes, bool split, bool shared, int ctas, int threads,
                             cudaStream_t stream);
 int propagateSmemBytes(const StepParams& p, int lanes, int threads);
+// 0 where the shape does not fit an SM
 int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, int threads, int smem);
 // The compiled instantiation's attributes (maxThreadsPerBlock, numRegs,
-// localSizeBytes): the launch shape never asks for more threads than the
-// instantiation accepts.
+// sharedSizeBytes): the launch shape never asks for more threads than the
+// instantiation accepts, or more shared memory than its own leaves.
 cudaError_t propagateAttributes(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, cudaFuncAttributes* a);
 
 }  // namespace phop

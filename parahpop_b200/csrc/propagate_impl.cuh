@@ -459,12 +459,6 @@ static __device__ __noinline__ void tideAloneAccel(const Rec r, const double pos
 // ordered before the other's reads, and neither overwrites what the other may
 // still read.  Kernel, ten steps at degree 70: 33
 // objects 3.77 -> 2.04 ms, 1,000 4.28 -> 2.12, 4,000 4.81 -> 3.34.
-constexpr int kDuoPairs = 4;  // pairs of a CTA of kDeepThreads threads
-struct DuoMail {
-    double f[3], sec, gast;
-    int block, valid;
-    double rho;
-};
 struct Duo {
     DuoMail* mail;  // of the pair's objects, 32 / L
     int* quit;

@@ -114,9 +114,13 @@ cudaError_t PHOP_CAT(launchPropagate_, PHOP_SUFFIX)(const StepParams& p, size_t 
 int PHOP_CAT(occupancy_, PHOP_SUFFIX)(int lanes, int pair, int deep, int stream, int duo, int nrl, int threads, int smem) {
     return dispatch(lanes, pair, deep, stream, duo, nrl, 0, [&](auto shape) -> int {
         auto k = kernelOf<decltype(shape)>();
-        if (smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem);
+        if ((smem > 48 * 1024
+             && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+            || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess) {
+            cudaGetLastError();  // the answer is 0; the launch that follows reports errors of its own
+            return 0;
+        }
         return n;
     });
 }
