@@ -1584,8 +1584,8 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
 // threads at 255 registers), and for small batches the drag model on a second
 // warp.  Threads per CTA follow from the bound, shared
 // memory and the batch size (prepareStep).  The first batch of each class
-// (log2 of the batch size, time-grid mode, precision, pairing and bound
-// options) times a short probe of
+// (log2 of the batch size and the lane counts at which it fits one wave of warp
+// pairs, time-grid mode, precision, pairing and bound options) times a short probe of
 // every shape on scratch copies of the inputs and keeps the fastest; later
 // batches of the class reuse the choice.  A probe launch advances every
 // object by up to twelve steps, fewer for large batches so that one launch
@@ -1597,8 +1597,13 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
                        int64_t* launches) {
     int bucket = 0;
     while (bucket < 40 && (int64_t(1) << bucket) < base.n) ++bucket;
-    const int key = ((bucket * 4 + (shared ? 2 : 0) + (opt.split ? 1 : 0)) * 4 + (opt.pairSh + 1)) * 4
-                    + (opt.deepRegs + 1);
+    // the lane counts at which the batch fits one wave of warp pairs: within a
+    // class all batches do or none, so that no batch is given a pair shape
+    // another's size was timed for
+    int waves = 0;
+    for (int L = 1; L <= 16; L *= 2) waves += duoFits(base.n, L) ? 1 : 0;
+    const int key = (((bucket * 4 + (shared ? 2 : 0) + (opt.split ? 1 : 0)) * 4 + (opt.pairSh + 1)) * 4
+                     + (opt.deepRegs + 1)) * 8 + waves;
     auto it = tuned_.find(key);
     if (it != tuned_.end()) return it->second;
     if (base.stride != 0 && base.stride != base.n) {  // pools pin their lane count
