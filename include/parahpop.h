@@ -190,6 +190,12 @@ int phop_propagate_device_noalloc(phop_context* ctx, int64_t n, double* d_states
  *              1 = 256 threads a CTA with up to 255 registers a thread, 0 =
  *              320 (two lanes) or 384 (four lanes) threads with up to 168;
  *              -1 (default) = chosen by the autotuner (pinned lanes: 0)
+ *   "drag_warp"  NRLMSISE-00 on a second warp beside the rest of the force
+ *              model: 1 = wherever the shape has such a kernel (lane-group
+ *              pairs at one, two and four lanes; no pairs at eight and
+ *              sixteen), 0 = never, -1 (default) = autotuned for batches of
+ *              up to one wave (pinned lanes: never; server: slices of up to
+ *              one wave); the same results in every case
  *   "tile_wait_test"  1 = test of the tile-staging time-out: the staging
  *              barrier is armed but no copy issued, so every CTA's bounded
  *              wait runs out and the CTA reads the tile from global memory
@@ -260,6 +266,7 @@ typedef struct {
     int pair_sh;             /* the geopotential ran for lane-group pairs (two objects per lane) */
     int deep_registers;      /* the step kernel ran at its deep thread bound (256 threads, <= 255 registers) */
     int registers;           /* registers a thread of the step kernel instantiation used */
+    int kernel_form;         /* 1: the drag model ran on a second warp; + 2: the tile was streamed through rings */
 } phop_stats;
 
 int phop_last_stats(const phop_context* ctx, phop_stats* out);

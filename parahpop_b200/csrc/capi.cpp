@@ -257,6 +257,12 @@ int phop_set_option(phop_context* ctx, const char* key, double value) {
             return 1;
         }
         ctx->opt.deepRegs = (int)value;
+    } else if (k == "drag_warp") {
+        if (value != -1.0 && value != 0.0 && value != 1.0) {
+            ctx->error = "drag_warp must be -1 (by batch size), 0 or 1";
+            return 1;
+        }
+        ctx->opt.dragWarp = (int)value;
     } else if (k == "tile_wait_test") {
         ctx->opt.tileWaitTest = value != 0.0 ? 1 : 0;
     } else if (k == "split_fp64_degree") {
@@ -620,6 +626,7 @@ int phop_last_stats(const phop_context* ctx, phop_stats* out) {
     out->pair_sh = ctx->stats.pairSh ? 1 : 0;
     out->deep_registers = ctx->stats.deepRegs ? 1 : 0;
     out->registers = ctx->stats.registers;
+    out->kernel_form = (ctx->stats.duo ? 1 : 0) | (ctx->stats.streamTile ? 2 : 0);
     return 0;
 }
 

@@ -1602,8 +1602,8 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
     // another's size was timed for
     int waves = 0;
     for (int L = 1; L <= 16; L *= 2) waves += duoFits(base.n, L) ? 1 : 0;
-    const int key = (((bucket * 4 + (shared ? 2 : 0) + (opt.split ? 1 : 0)) * 4 + (opt.pairSh + 1)) * 4
-                     + (opt.deepRegs + 1)) * 8 + waves;
+    const int key = ((((bucket * 4 + (shared ? 2 : 0) + (opt.split ? 1 : 0)) * 4 + (opt.pairSh + 1)) * 4
+                     + (opt.deepRegs + 1)) * 8 + waves) * 4 + (opt.dragWarp + 1);
     auto it = tuned_.find(key);
     if (it != tuned_.end()) return it->second;
     if (base.stride != 0 && base.stride != base.n) {  // pools pin their lane count
@@ -1646,7 +1646,8 @@ int Engine::tunedShape(const StepParams& base, const RunOptions& opt, bool share
         if (opt.pairSh < 0 && L <= 4 && pair && columns_ == 0) continue;
         if (opt.pairSh < 0 && L <= 4 && !pair && columns_ > 16) continue;
         if (opt.deepRegs < 0 && hasDeepShape(L) && !deep) continue;
-        if (duo && (!hasDuo(L, pair) || !duoFits(n, L))) continue;
+        const bool duoShape = hasDuo(L, pair) && nrlDrag();
+        if (opt.dragWarp < 0 ? duo && !(duoShape && duoFits(n, L)) : duo != (opt.dragWarp && duoShape ? 1 : 0)) continue;
         RunOptions o = opt;
         o.pairSh = pair;
         o.deepRegs = deep;
@@ -1750,6 +1751,7 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
     PHOP_CUDA(cudaMemsetAsync(dCtl, 0, 4 * sizeof(int), stream));
     PHOP_CUDA(cudaEventRecord(eTuned, stream));  // end of the epoch records
     RunOptions o = opt;
+    o.duo = opt.dragWarp > 0;
     int L = opt.lanes;
     if (L <= 0) {
         const int code = tunedShape(p, opt, shared, stream, &launches);
@@ -1792,6 +1794,8 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
         stats->tileInSmem = shape.smemTile;
         stats->pairSh = p.pairSh != 0;
         stats->deepRegs = p.deepRegs != 0;
+        stats->duo = p.duo != 0;
+        stats->streamTile = p.streamTile != 0;
         stats->registers = shape.registers;
     }
 }

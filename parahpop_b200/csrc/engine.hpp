@@ -130,6 +130,8 @@ struct RunStats {
     bool pairSh = false;           // the geopotential of lane-group pairs was used
     bool deepRegs = false;         // the deep thread bound (256 threads, 255 registers) was used
     int registers = 0;             // registers a thread of the step kernel used
+    bool duo = false;              // the drag model ran on a second warp
+    bool streamTile = false;       // the coefficient tile was streamed through rings
     int64_t tileFallbacks = 0;     // CTAs that read the tile from global memory after a staging time-out
 };
 
@@ -149,6 +151,8 @@ struct RunOptions {
                           // -1 autotuned with the lane count (pinned lanes: on up to 4 lanes)
     int deepRegs = -1;    // thread bound at 2 and 4 lanes: 1 deep (256 threads, 255 registers), 0 wide
                           // (320 / 384 threads, 168 registers), -1 autotuned (pinned lanes: wide)
+    int dragWarp = -1;    // the drag model on a second warp: 1 wherever a shape has it, 0 never, -1 by batch size
+                          // (autotuned; pinned lanes: never; server slices: up to one wave)
     int duo = 0;          // small batches: the drag model on a second warp (StepParams::duo); the autotuner's
                           // choice (pinned lanes: 0)
     // trajectory records of a uniform batch: device buffer of

@@ -301,10 +301,13 @@ int Server::step() {
         p.workCounter = ctl_;
         p.errorFlag = ctl_ + 1;
         PHOP_SCUDA(cudaEventRecord(ev0_, stream_));
-        // a slice of one wave runs its drag model on second warps (the same
-        // results bit for bit)
+        // a slice of one wave runs its drag model on second warps.  Which kernel
+        // an object meets then depends on what shares its slice; the two give
+        // the same bits as built (the terms outside the field are contracted
+        // by the compiler in each), which the GPU tests hold over force
+        // models, populations and tiles
         RunOptions o = opt_;
-        o.duo = o.deepRegs > 0 && engine_.duoFits(nAct, lanes_);
+        o.duo = o.dragWarp >= 0 ? o.dragWarp : o.deepRegs > 0 && engine_.duoFits(nAct, lanes_);
         engine_.launchStep(p, lanes_, o, false, stream_);
         PHOP_SCUDA(cudaEventRecord(ev1_, stream_));
         PHOP_SCUDA(cudaEventSynchronize(ev1_));
