@@ -293,14 +293,15 @@ static __device__ __forceinline__ double nrlDensityBody(const DevEnv& e, NrlTime
     const double rho2 = f[0] * f[0] + f[1] * f[1], r2 = rho2 + f[2] * f[2];
     if (!(r2 > 0.0)) return NAN;
     const double radius = e.earthRadius;
-    // the ellipsoid lies inside the sphere of its equatorial radius: above the
-    // cut-off from there is above it everywhere
+    // an oblate ellipsoid lies inside the sphere of its equatorial radius:
+    // above the cut-off from there is above it everywhere
+    const bool oblate = e.flattening >= 0.0 && e.flattening < 1.0;
     const double clear = radius + e.nrlHcutoff;
-    if (e.nrlHcutoff >= 0.0 && r2 > clear * clear && r2 < 1e30) return 0.0;
+    if (oblate && e.nrlHcutoff >= 0.0 && r2 > clear * clear && r2 < 1e30) return 0.0;
     const double e2 = e.flattening * (2.0 - e.flattening);
     const double rho = sqrt(rho2);
-    double dz, zdz, nn = radius, nh = 0.0;
-    {
+    double dz = e2 * f[2], zdz, nn = radius, nh = 0.0;
+    if (oblate) {
         // start from Bowring's latitude (Survey Review 23(181), 1976), off by
         // less than 1e-11 rad in orbit, so that the fixed point below ends
         // after one pass instead of five (with the angle rotations below, a
