@@ -189,7 +189,8 @@ int phop_propagate_device_noalloc(phop_context* ctx, int64_t n, double* d_states
  *   "deep_registers"  thread bound of the step kernel at two and four lanes:
  *              1 = 256 threads a CTA with up to 255 registers a thread, 0 =
  *              320 (two lanes) or 384 (four lanes) threads with up to 168;
- *              -1 (default) = chosen by the autotuner (pinned lanes: 0)
+ *              -1 (default) = chosen by the autotuner (pinned lanes: 0, or 1
+ *              where the tile does not fit shared memory and 1 streams it)
  *   "drag_warp"  NRLMSISE-00 on a second warp beside the rest of the force
  *              model: 1 = wherever the shape has such a kernel (lane-group
  *              pairs at one, two and four lanes; no pairs at eight and

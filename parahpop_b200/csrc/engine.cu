@@ -1529,12 +1529,23 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     };
     // "tile_smem" = 0 asks for reads through L1, and the FP64 floor of the
     // split form lets a warp's objects part in the row loop: no stream
-    const bool mayStream = opt.tileSmem != 0 && (p.duo ? L <= 4 : hasStream(L, p.deepRegs)) && tile.nblocks > 0
-                           && p.splitRadius == 0.0;
-    const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
-                      * (32 * halves);
-    const StepRoom room = stepRoom(maxSmem_, attributes(0).smem, mayStream ? attributes(1).smem : 0, tile.bytes, L,
-                                   p.duo != 0, bound, opt.tileSmem != 0, mayStream);
+    const auto boundOf = [&]() {
+        return std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
+               * (32 * halves);
+    };
+    const auto roomOf = [&](bool stream) {
+        return stepRoom(maxSmem_, attributes(0).smem, stream ? attributes(1).smem : 0, tile.bytes, L, p.duo != 0,
+                        boundOf(), opt.tileSmem != 0, stream);
+    };
+    const bool wouldStream = opt.tileSmem != 0 && tile.nblocks > 0 && p.splitRadius == 0.0;
+    // with lanes pinned and no bound asked for, the wide kernel unless its
+    // tile would be read from global memory, where the deep kernel streams it
+    // (10^4 LEO objects x 10 steps, degree 120 FP64, two lanes 44.8 -> 18.6
+    // ms, 41.8 with the smaller rows of the spherical-component sums)
+    if (opt.deepRegs < 0 && hasDeepShape(L) && !p.duo && wouldStream && !roomOf(false).staged) p.deepRegs = 1;
+    const bool mayStream = wouldStream && (p.duo ? L <= 4 : hasStream(L, p.deepRegs));
+    const int bound = boundOf();
+    const StepRoom room = roomOf(mayStream);
     p.useSmemTile = room.staged;
     p.streamTile = room.streamed;
     // never more threads than the compiled instantiation accepts (its

@@ -150,7 +150,8 @@ struct RunOptions {
     int pairSh = -1;      // geopotential of lane-group pairs (packed FP32 in split precision): 1 on, 0 off,
                           // -1 autotuned with the lane count (pinned lanes: on up to 4 lanes)
     int deepRegs = -1;    // thread bound at 2 and 4 lanes: 1 deep (256 threads, 255 registers), 0 wide
-                          // (320 / 384 threads, 168 registers), -1 autotuned (pinned lanes: wide)
+                          // (320 / 384 threads, 168 registers), -1 autotuned (pinned lanes: wide, or deep
+                          // where the tile does not fit shared memory)
     int dragWarp = -1;    // the drag model on a second warp: 1 wherever a shape has it, 0 never, -1 by batch size
                           // (autotuned; pinned lanes: never; server slices: up to one wave)
     int duo = 0;          // small batches: the drag model on a second warp (StepParams::duo); the autotuner's

@@ -201,13 +201,29 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.lowDeg = lowDeg;
     sp.workCounter = ctl;
     sp.errorFlag = ctl + 1;
-    const int threadsReq = std::min(opt.threads > 0 ? opt.threads : 512, maxStepThreads(L));
-    const int tileBytes = (int)ht.bytes.size();
-    const auto fit = [&](int bytes) { return (maxSmem_ - 1024 - bytes) / kStageBytes * L / 32 * 32; };
-    sp.useSmemTile = opt.tileSmem != 0 && tileBytes + 1024 <= maxSmem_ && fit(tileBytes) >= 64;
-    const int threads = std::min(threadsReq, fit(sp.useSmemTile ? tileBytes : 0));
+    // the wide kernel, or the streaming one where the tile does not fit shared
+    // memory (prepareStep has the figures)
+    const auto roomOf = [&](int stream) {
+        cudaFuncAttributes a{};
+        check(propagateAttributes(L, opt.split, true, 0, sp.deepRegs, stream, 0, sp.nrl, &a));
+        const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, sp.deepRegs));
+        StepRoom r = stepRoom(maxSmem_, (int)a.sharedSizeBytes, (int)a.sharedSizeBytes, sp.tileBytes, L, false, bound,
+                              opt.tileSmem != 0, stream != 0);
+        r.threads = std::min(bound, r.threads);
+        return r;
+    };
+    StepRoom room = roomOf(0);
+    if (!room.staged && opt.tileSmem != 0 && sp.nblocks > 0 && hasStream(L, 1)) {
+        sp.deepRegs = hasDeepShape(L);
+        room = roomOf(1);
+    }
+    sp.useSmemTile = room.staged;
+    sp.streamTile = room.streamed;
+    const int threads = room.threads;
     const int smem = propagateSmemBytes(sp, L, threads);
-    int perSm = opt.ctasPerSm > 0 ? opt.ctasPerSm : propagateMaxCtasPerSm(L, opt.split, true, 0, 0, 0, 0, sp.nrl, threads, smem);
+    int perSm = opt.ctasPerSm > 0 ? opt.ctasPerSm
+                                  : propagateMaxCtasPerSm(L, opt.split, true, 0, sp.deepRegs, sp.streamTile, 0, sp.nrl,
+                                                          threads, smem);
     if (perSm <= 0) perSm = 1;
     const int64_t groups = (n + (32 / L) - 1) / (32 / L);
     const int64_t need = (groups + threads / 32 - 1) / (threads / 32);
