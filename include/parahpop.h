@@ -180,7 +180,8 @@ int phop_propagate_device_noalloc(phop_context* ctx, int64_t n, double* d_states
  *              launches
  *   "tile_smem"  1 (default) = stage the coefficient tile in shared memory
  *              when it fits, or stream it through rings there (one lane per
- *              object, and the deep thread bound); 0 = read it through L1
+ *              object, and the deep thread bound), or stage its first blocks;
+ *              0 = read it through L1
  *   "pair_sh"  geopotential of lane-group pairs, two objects per lane
  *              (each coefficient loaded from shared memory serves both;
  *              packed FP32 in split precision; at one, two or four lanes
@@ -267,7 +268,8 @@ typedef struct {
     int pair_sh;             /* the geopotential ran for lane-group pairs (two objects per lane) */
     int deep_registers;      /* the step kernel ran at its deep thread bound (256 threads, <= 255 registers) */
     int registers;           /* registers a thread of the step kernel instantiation used */
-    int kernel_form;         /* 1: the drag model ran on a second warp; + 2: the tile was streamed through rings */
+    int kernel_form;         /* 1: the drag model ran on a second warp; + 2: the tile was streamed through rings;
+                              * + 4: its first blocks were staged in shared memory */
 } phop_stats;
 
 int phop_last_stats(const phop_context* ctx, phop_stats* out);

@@ -626,7 +626,7 @@ int phop_last_stats(const phop_context* ctx, phop_stats* out) {
     out->pair_sh = ctx->stats.pairSh ? 1 : 0;
     out->deep_registers = ctx->stats.deepRegs ? 1 : 0;
     out->registers = ctx->stats.registers;
-    out->kernel_form = (ctx->stats.duo ? 1 : 0) | (ctx->stats.streamTile ? 2 : 0);
+    out->kernel_form = (ctx->stats.duo ? 1 : 0) | (ctx->stats.streamTile ? 2 : 0) | (ctx->stats.tileInPart ? 4 : 0);
     return 0;
 }
 

@@ -1529,12 +1529,14 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     };
     // "tile_smem" = 0 asks for reads through L1, and the FP64 floor of the
     // split form lets a warp's objects part in the row loop: no stream
+    const TileShape tileShape{tile.bytes, tile.nblocks, p.pairSh ? 2 * L : L, host_.shDegree,
+                              opt.split ? lowDeg : host_.shDegree};
     const auto boundOf = [&]() {
         return std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, p.deepRegs, p.duo)) / (32 * halves)
                * (32 * halves);
     };
     const auto roomOf = [&](bool stream) {
-        return stepRoom(maxSmem_, attributes(0).smem, stream ? attributes(1).smem : 0, tile.bytes, L, p.duo != 0,
+        return stepRoom(maxSmem_, attributes(0).smem, stream ? attributes(1).smem : 0, tileShape, L, p.duo != 0,
                         boundOf(), opt.tileSmem != 0, stream);
     };
     const bool wouldStream = opt.tileSmem != 0 && tile.nblocks > 0 && p.splitRadius == 0.0;
@@ -1546,7 +1548,8 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     const bool mayStream = wouldStream && (p.duo ? L <= 4 : hasStream(L, p.deepRegs));
     const int bound = boundOf();
     const StepRoom room = roomOf(mayStream);
-    p.useSmemTile = room.staged;
+    p.useSmemTile = room.stagedBytes > 0;
+    p.stagedBytes = room.stagedBytes;
     p.streamTile = room.streamed;
     // never more threads than the compiled instantiation accepts (its
     // register count times the threads must fit the SM's register file)
@@ -1582,7 +1585,7 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     shape.lanes = L;
     shape.threads = threads;
     shape.ctas = (int)std::max<int64_t>(1, std::min<int64_t>(slots, need));
-    shape.smemTile = p.useSmemTile != 0;
+    shape.smemTile = room.staged;
     shape.registers = registers;
     shape.fits = fits;
     return shape;
@@ -1807,6 +1810,7 @@ void Engine::runKernel(int64_t n, double* dState, const double* dBc, const doubl
         stats->deepRegs = p.deepRegs != 0;
         stats->duo = p.duo != 0;
         stats->streamTile = p.streamTile != 0;
+        stats->tileInPart = p.useSmemTile && p.stagedBytes < p.tileBytes;
         stats->registers = shape.registers;
     }
 }

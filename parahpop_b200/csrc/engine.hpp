@@ -132,6 +132,7 @@ struct RunStats {
     int registers = 0;             // registers a thread of the step kernel used
     bool duo = false;              // the drag model ran on a second warp
     bool streamTile = false;       // the coefficient tile was streamed through rings
+    bool tileInPart = false;       // its first blocks were staged in shared memory
     int64_t tileFallbacks = 0;     // CTAs that read the tile from global memory after a staging time-out
 };
 

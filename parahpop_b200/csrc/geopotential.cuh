@@ -123,7 +123,7 @@ extern __shared__ __align__(128) unsigned char g_smem[];
 struct TileRef {
     const void* global;
     int nblocks;
-    bool staged;
+    int staged;  // 16-byte chunks staged: whole blocks from the tile's start
 };
 
 // The stream of a tile too large for shared memory: the warp copies it, stage
@@ -249,7 +249,7 @@ static __device__ __forceinline__ void fieldRows(const TileRef& tile, TileStream
                                                  Lanes<T, K>& q1, Lanes<T, K> (&S)[6]) {
     using Chunk = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
     constexpr int kChunks = PairRows<T>::kChunks, kStep = kChunks * W;
-    if (MODE == TileRead::kShared && tile.staged) {
+    if (MODE == TileRead::kShared && chunk < tile.staged) {
         const Chunk* tp = (const Chunk*)g_smem + chunk + pj;
 #pragma unroll 2
         for (int i = 0; i < pairs; ++i, tp += kStep) {
@@ -280,7 +280,7 @@ static __device__ __forceinline__ void fieldRows(const TileRef& tile, TileStream
         return;
     }
     const Chunk* __restrict__ tp =
-        (const Chunk*)(MODE == TileRead::kGeneric && tile.staged ? (const void*)g_smem : tile.global) + chunk + pj;
+        (const Chunk*)(MODE == TileRead::kGeneric && chunk < tile.staged ? (const void*)g_smem : tile.global) + chunk + pj;
     for (int i = 0; i < pairs; ++i, tp += kStep) {
         PairRows<T> r;
         r.template load<W>(tp);

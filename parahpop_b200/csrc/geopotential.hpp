@@ -79,6 +79,17 @@ PHOP_GEO_HD int rowPairs32(int M, int N, int lowDeg) {
     return rows > 0 ? (rows + 1) / 2 : 0;
 }
 
+// Bytes of the first blocks of a tile that fit `limit`
+inline int leadingBlocks(int nblocks, int W, int N, int lowDeg, int limit) {
+    int bytes = 0;
+    for (int b = 0; b < nblocks; ++b) {
+        const int next = (rowPairs64(b * W, N, lowDeg) * kChunks64 + rowPairs32(b * W, N, lowDeg) * kChunks32) * W * 16;
+        if (next > limit - bytes) break;
+        bytes += next;
+    }
+    return bytes;
+}
+
 // A tile too large for shared memory is streamed through a ring of
 // kRingStages stages per warp.
 constexpr int kStageChunks = 128;  // 16-byte chunks of a stage: four a lane

@@ -203,11 +203,12 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
     sp.errorFlag = ctl + 1;
     // the wide kernel, or the streaming one where the tile does not fit shared
     // memory (prepareStep has the figures)
+    const TileShape tileShape{sp.tileBytes, sp.nblocks, L, host_.shDegree, opt.split ? lowDeg : host_.shDegree};
     const auto roomOf = [&](int stream) {
         cudaFuncAttributes a{};
         check(propagateAttributes(L, opt.split, true, 0, sp.deepRegs, stream, 0, sp.nrl, &a));
         const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, sp.deepRegs));
-        StepRoom r = stepRoom(maxSmem_, (int)a.sharedSizeBytes, (int)a.sharedSizeBytes, sp.tileBytes, L, false, bound,
+        StepRoom r = stepRoom(maxSmem_, (int)a.sharedSizeBytes, (int)a.sharedSizeBytes, tileShape, L, false, bound,
                               opt.tileSmem != 0, stream != 0);
         r.threads = std::min(bound, r.threads);
         return r;
@@ -217,7 +218,8 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
         sp.deepRegs = hasDeepShape(L);
         room = roomOf(1);
     }
-    sp.useSmemTile = room.staged;
+    sp.useSmemTile = room.stagedBytes > 0;
+    sp.stagedBytes = room.stagedBytes;
     sp.streamTile = room.streamed;
     const int threads = room.threads;
     const int smem = propagateSmemBytes(sp, L, threads);

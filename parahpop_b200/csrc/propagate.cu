@@ -95,7 +95,7 @@ void launchRecordPairs(const EpochRecord* grid, int64_t count, double2* pairs, c
 }
 
 int propagateSmemBytes(const StepParams& p, int lanes, int threads) {
-    return (p.useSmemTile ? p.tileBytes : p.streamTile ? threads / (p.duo ? 64 : 32) * kRingBytes : 0) + kStageBytes * (threads / (p.duo ? 2 : 1) / lanes);
+    return (p.useSmemTile ? p.stagedBytes : p.streamTile ? threads / (p.duo ? 64 : 32) * kRingBytes : 0) + kStageBytes * (threads / (p.duo ? 2 : 1) / lanes);
 }
 
 int propagateMaxCtasPerSm(int lanes, bool split, bool shared, int pair, int deep, int stream, int duo, int nrl, int threads, int smem) {

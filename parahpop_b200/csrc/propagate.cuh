@@ -93,6 +93,7 @@ struct StepParams {
     int nblocks64;
     double splitRadius;     // split precision: radius (km) below which the tile part stays FP64; 0 = none
     int useSmemTile;
+    int stagedBytes;        // of the tile in shared memory: all, or the first blocks (stepRoom)
     int streamTile;         // the tile streamed through rings in shared memory (hasStream shapes)
     int pairSh;             // the geopotential of lane-group pairs (tile built for 2L lanes)
     int duo;                // warps in pairs, the drag model on the second (hasDuo shapes)
@@ -143,27 +144,44 @@ struct DuoMail {
 };
 struct StepRoom {
     int threads = 0;          // most threads the shared memory has room for
-    bool staged = false, streamed = false;
+    bool staged = false, streamed = false;  // the whole tile in shared memory; through rings there
+    int stagedBytes = 0;      // whole tile, or its first blocks
 };
 // A tile that does not fit, or leaves room for fewer than three quarters of
 // the threads, is streamed through a ring per warp where the kernel can (a
 // streamed row costs about a fifth more than a staged one).  maxSmem: what a
 // CTA may use in all; ownStaged, ownStreamed: what the kernels with and
-// without a stream hold by themselves; bound: the threads asked for.
-inline StepRoom stepRoom(int maxSmem, int ownStaged, int ownStreamed, int tileBytes, int lanes, bool duo, int bound,
+// without a stream hold by themselves; bound: the threads asked for.  Where
+// it neither fits nor streams (eight and sixteen lanes, the wide bound at two
+// and four), its first blocks are staged beside the stage accelerations and
+// the rest is read from global memory: with the rows of the solid harmonics a
+// tile of eight or sixteen lanes fits to FP64 degree 84 or 80, with the former
+// rows to 92 or 89, and read from global memory throughout, the field of one
+// object at degree 88 took 3.4 ms for ten steps at its best shape; 2.08 with
+// the former rows, 1.85 with the first blocks staged.
+struct TileShape {
+    int bytes, nblocks, W, degree, lowDeg;
+};
+inline StepRoom stepRoom(int maxSmem, int ownStaged, int ownStreamed, const TileShape& tile, int lanes, bool duo, int bound,
                          bool mayStage, bool mayStream) {
     const int halves = duo ? 2 : 1;  // half of a duo CTA's warps hold objects
     const auto room = [&](int own) { return maxSmem - (own > 1024 ? own : 1024); };
     const auto fit = [&](int bytes) {
         return bytes < room(ownStaged) ? (room(ownStaged) - bytes) / kStageBytes * lanes / 32 * 32 * halves : 0;
     };
-    const int staged = mayStage ? fit(tileBytes) : 0;
+    const int staged = mayStage ? fit(tile.bytes) : 0;
     const int streamed = mayStream ? room(ownStreamed) / (kRingBytes + kStageBytes * (32 / lanes)) * 32 * halves : 0;
     const auto most = [&](int t) { return t < bound ? t : bound; };
     StepRoom r;
     r.streamed = mayStream && most(staged) < most(streamed) * 3 / 4;
     r.staged = !r.streamed && staged >= 64;
     r.threads = r.staged ? staged : r.streamed ? streamed : fit(0);
+    if (r.staged) {
+        r.stagedBytes = tile.bytes;
+    } else if (mayStage && !r.streamed) {
+        r.stagedBytes = leadingBlocks(tile.nblocks, tile.W, tile.degree, tile.lowDeg,
+                                      room(ownStaged) - kStageBytes * (most(r.threads) / halves / lanes));
+    }
     return r;
 }
 

@@ -567,7 +567,7 @@ static __device__ __forceinline__ void accelerations(const StepParams& p, const 
             if (!PAIR && sizeof(T) == 4 && p.splitRadius > 0.0
                 && bx * bx + by * by + bz * bz < p.splitRadius * p.splitRadius) {
                 TileStream<L> none;
-                fieldAccel<L, 1, double, TileRead::kGeneric>(p, TileRef{p.tile64, p.nblocks64, false}, none, r, bx, by, bz, a);
+                fieldAccel<L, 1, double, TileRead::kGeneric>(p, TileRef{p.tile64, p.nblocks64, 0}, none, r, bx, by, bz, a);
             } else {
                 fieldAccel<L, PAIR ? 2 : 1, T, MODE>(p, tile, stream, r, bx, by, bz, a);
             }
@@ -806,7 +806,7 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
                               : MAXT <= kDeepThreads ? TileRead::kShared
                                                      : TileRead::kGeneric;
     constexpr int NA = Axes<L>::N;
-    TileRef tile{p.tile, p.nblocks, false};
+    TileRef tile{p.tile, p.nblocks, 0};
     int kOffset = 0;
     if (!SHARED_GRID && !p.gridPairs) {  // per-object time needs the batch's record grid
         if (threadIdx.x == 0) atomicExch(p.errorFlag, 3);
@@ -814,11 +814,11 @@ __global__ void __launch_bounds__(MAXT, 1) propagateKernel(const __grid_constant
     }
     if (!STREAM && p.useSmemTile) {
         const bool test = p.tileWaitTest != 0;
-        if (stageTile(g_smem, p.tile, p.tileBytes, !test, test ? 4096L : (1L << 24)))
-            tile.staged = true;
+        if (stageTile(g_smem, p.tile, p.stagedBytes, !test, test ? 4096L : (1L << 24)))
+            tile.staged = p.stagedBytes / 16;
         else if (threadIdx.x == 0 && p.tileFallbacks)
             atomicAdd(p.tileFallbacks, 1);  // this CTA reads the tile from global memory
-        kOffset = p.tileBytes;
+        kOffset = p.stagedBytes;
     }
     // main warps of the CTA and this warp's place among them
     const int warps = (int)(blockDim.x / 32) / (DUO ? 2 : 1), warp = (int)(threadIdx.x / 32) / (DUO ? 2 : 1);

@@ -8,13 +8,13 @@
 
 using namespace phop;
 
-static int tileBytes(int N, int W, bool split) {
+static TileShape tileOf(int N, int W, bool split) {
     const int low = split ? (N > 80 ? kSplitFp64DegreeHigh : kSplitFp64Degree) : N, columns = N + 2;
     long b = 0;
     for (int k = 0; k < (columns + W - 1) / W; ++k)
         b += ((long)rowPairs64(k * W, N, low) * kChunks64 + (long)rowPairs32(k * W, N, low) * kChunks32) * W * 16;
     const int stage = kStageChunks * 16;
-    return (int)((b + stage - 1) / stage * stage);
+    return TileShape{(int)((b + stage - 1) / stage * stage), (columns + W - 1) / W, W, N, low};
 }
 
 int main() {
@@ -31,14 +31,14 @@ int main() {
                         const int own = (8 + mail + 127) / 128 * 128;
                         const bool mayStream = duo ? L <= 4 : hasStream(L, deep);
                         for (int N = 1; N <= 400; ++N) {
-                            const int bytes = tileBytes(N, pair ? 2 * L : L, split != 0);
+                            const TileShape tile = tileOf(N, pair ? 2 * L : L, split != 0);
                             const int bound = stepThreadBound(L, deep, duo), halves = duo ? 2 : 1;
-                            const StepRoom r = stepRoom(kMax, own, own, bytes, L, duo != 0, bound, true, mayStream);
+                            const StepRoom r = stepRoom(kMax, own, own, tile, L, duo != 0, bound, true, mayStream);
                             const int threads = std::min(bound, r.threads);
-                            const int dynamic = (r.staged ? bytes : r.streamed ? threads / (32 * halves) * kRingBytes : 0)
+                            const int dynamic = (r.stagedBytes > 0 ? r.stagedBytes : r.streamed ? threads / (32 * halves) * kRingBytes : 0)
                                                 + kStageBytes * (threads / halves / L);
                             ++shapes;
-                            over += own + dynamic > kMax;
+                            over += own + dynamic > kMax || (r.stagedBytes > 0 && (r.streamed || r.stagedBytes > tile.bytes || r.stagedBytes % 16));
                             none += threads < 32 * halves;
                             most = std::max(most, own + dynamic);
                         }

@@ -29,7 +29,7 @@ def both(prop, run, streamed=None):
         form = prop.stats()["kernel_form"]
         assert form & 1 == duo, form
         if streamed is not None:
-            assert form >> 1 == int(streamed), form
+            assert (form >> 1) & 1 == int(streamed), form
     assert np.isfinite(out[0]).all()
     np.testing.assert_array_equal(out[0], out[1])
 

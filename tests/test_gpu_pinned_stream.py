@@ -36,12 +36,34 @@ def test_pinned_lanes(tmp_path, degree, split):
                 assert s["deep_registers"] == (lanes > 1 and degree == 120)
                 assert s["kernel_form"] == (2 if degree == 120 else 0)
             if deep == 0 and lanes > 1:
-                assert s["kernel_form"] == 0 and s["deep_registers"] == 0
+                assert s["kernel_form"] == (4 if degree == 120 else 0) and s["deep_registers"] == 0
         assert np.isfinite(out[-1]).all()
         np.testing.assert_array_equal(out[-1], out[1 if degree == 120 else 0])
 
 
-@pytest.mark.parametrize("lanes", [1, 2, 4, 8])
+@pytest.mark.parametrize("split,degree", [(False, 88), (False, 120), (True, 120)])
+@pytest.mark.parametrize("lanes,duo", [(2, 0), (4, 0), (8, 0), (16, 0), (8, 1), (16, 1)])
+def test_first_blocks_staged(tmp_path, lanes, duo, split, degree):
+    """The staged blocks are those of global memory: the same bits, on both
+    time grids, with part-filled warps and several items a warp."""
+    cfg = config(tmp_path, degree)
+    for n in (1, 37, 20000 // lanes):
+        pop = S.population_leo(n, seed=n, screen_duration=240.0)
+        for epochs in (pop.epochs, pop.epochs + np.linspace(0.001, 0.01, n)):
+            got = []
+            for smem in (1, 0):
+                p = api.Propagator(cfg, lanes=lanes, split=split)
+                for key, value in (("tile_smem", smem), ("deep_registers", 0), ("drag_warp", duo)):
+                    p.set_option(key, value)
+                got.append(p.propagate(epochs, pop.states, pop.mass, pop.drag_area, pop.srp_area, pop.cd, pop.cr)[1])
+                s = p.stats()
+                assert s["kernel_form"] == duo + (4 if smem else 0) and s["tile_in_smem"] == 0
+                p.close()
+            assert np.isfinite(got[0]).all()
+            np.testing.assert_array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("lanes", [1, 2, 4, 8, 16])
 def test_noalloc(tmp_path, lanes):
     """To the entry points' parity tolerance, 1 mm and 1e-6 m/s; a refused
     call's limits are as before."""
