@@ -1537,7 +1537,7 @@ Engine::LaunchShape Engine::prepareStep(StepParams& p, int L, const RunOptions& 
     };
     const auto roomOf = [&](bool stream) {
         return stepRoom(maxSmem_, attributes(0).smem, stream ? attributes(1).smem : 0, tileShape, L, p.duo != 0,
-                        boundOf(), opt.tileSmem != 0, stream);
+                        boundOf(), opt.tileSmem != 0, stream, hasPart(L, p.deepRegs || p.duo));
     };
     const bool wouldStream = opt.tileSmem != 0 && tile.nblocks > 0 && p.splitRadius == 0.0;
     // with lanes pinned and no bound asked for, the wide kernel unless its

@@ -209,7 +209,7 @@ void Engine::propagateNoAlloc(int64_t n, double* dState, const double* dBc, cons
         check(propagateAttributes(L, opt.split, true, 0, sp.deepRegs, stream, 0, sp.nrl, &a));
         const int bound = std::min(opt.threads > 0 ? opt.threads : 512, stepThreadBound(L, sp.deepRegs));
         StepRoom r = stepRoom(maxSmem_, (int)a.sharedSizeBytes, (int)a.sharedSizeBytes, tileShape, L, false, bound,
-                              opt.tileSmem != 0, stream != 0);
+                              opt.tileSmem != 0, stream != 0, hasPart(L, sp.deepRegs));
         r.threads = std::min(bound, r.threads);
         return r;
     };

@@ -124,6 +124,9 @@ __host__ __device__ constexpr bool hasDeepShape(int lanes) { return lanes == 2 |
 __host__ __device__ constexpr bool hasStream(int lanes, int deep) {
     return lanes == 1 || (deep && hasDeepShape(lanes));
 }
+// shapes that can hold the first blocks of a tile and read the rest from
+// global memory
+__host__ __device__ constexpr bool hasPart(int lanes, int deep) { return lanes >= 8 || (hasDeepShape(lanes) && !deep); }
 // shapes with the drag model on a second warp, at the deep bound: two lane
 // groups sharing columns up to four lanes, one object a lane at eight and
 // sixteen
@@ -163,7 +166,7 @@ struct TileShape {
     int bytes, nblocks, W, degree, lowDeg;
 };
 inline StepRoom stepRoom(int maxSmem, int ownStaged, int ownStreamed, const TileShape& tile, int lanes, bool duo, int bound,
-                         bool mayStage, bool mayStream) {
+                         bool mayStage, bool mayStream, bool mayPart) {
     const int halves = duo ? 2 : 1;  // half of a duo CTA's warps hold objects
     const auto room = [&](int own) { return maxSmem - (own > 1024 ? own : 1024); };
     const auto fit = [&](int bytes) {
@@ -178,7 +181,7 @@ inline StepRoom stepRoom(int maxSmem, int ownStaged, int ownStreamed, const Tile
     r.threads = r.staged ? staged : r.streamed ? streamed : fit(0);
     if (r.staged) {
         r.stagedBytes = tile.bytes;
-    } else if (mayStage && !r.streamed) {
+    } else if (mayStage && mayPart && !r.streamed) {
         r.stagedBytes = leadingBlocks(tile.nblocks, tile.W, tile.degree, tile.lowDeg,
                                       room(ownStaged) - kStageBytes * (most(r.threads) / halves / lanes));
     }

@@ -33,7 +33,7 @@ int main() {
                         for (int N = 1; N <= 400; ++N) {
                             const TileShape tile = tileOf(N, pair ? 2 * L : L, split != 0);
                             const int bound = stepThreadBound(L, deep, duo), halves = duo ? 2 : 1;
-                            const StepRoom r = stepRoom(kMax, own, own, tile, L, duo != 0, bound, true, mayStream);
+                            const StepRoom r = stepRoom(kMax, own, own, tile, L, duo != 0, bound, true, mayStream, hasPart(L, deep || duo));
                             const int threads = std::min(bound, r.threads);
                             const int dynamic = (r.stagedBytes > 0 ? r.stagedBytes : r.streamed ? threads / (32 * halves) * kRingBytes : 0)
                                                 + kStageBytes * (threads / halves / L);
