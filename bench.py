@@ -42,6 +42,7 @@ sys.path.insert(0, str(ROOT))
 METRIC = "object-steps/s full-force at ≤1 cm vs FP64 oracle; p50/p99 request latency"
 SH_FLOP_PER_TERM = 18  # algorithmic FLOPs per row of the field's column sums: a recurrence step and six sums
 SH_EVALUATIONS = 12.0  # force evaluations per step (the thirteenth stage serves only the error estimate)
+SPLIT_FP64_MARGIN = 11  # FP64 degrees of the split form beyond its low part
 SPLIT_TOL_M = 1e-2
 FP64_TOL_M = 1e-3
 
@@ -58,10 +59,10 @@ def sh_flops_per_object_step(degree: int) -> float:
 # captures (profiles/): the state is read once and written once per launch
 # (~100 B per object); the rest is local memory written back from L2 and the
 # epoch-record grid.  c3: the split form's kernel at one lane with lane-group
-# pairs, 10^5 objects x 24 steps (17.09 + 6.43 GB over 2,391,620
+# pairs, 10^5 objects x 24 steps (17.42 + 6.36 GB over 2,391,620
 # object-steps); the other workloads have no capture of the current kernel
 # (null).
-NCU_BYTES_PER_OBJECT_STEP = {"c3": (17.090873e9 + 6.427766e9) / 2_391_620, "c1": None, "c2": None}
+NCU_BYTES_PER_OBJECT_STEP = {"c3": (17.419499e9 + 6.356519e9) / 2_391_620, "c1": None, "c2": None}
 
 
 def dist_env():
@@ -622,7 +623,7 @@ def main():
         flops = sh_flops_per_object_step(degree) * r["object_steps"]
         achieved = flops / (r["kernel_ms"] * 1e-3) * 1e-12
         if head == "split":
-            low = args.split_degree or (24 if degree > 80 else 20)  # the library's default by field degree
+            low = min(degree, (args.split_degree or (24 if degree > 80 else 20)) + SPLIT_FP64_MARGIN)  # library default
             f64 = SH_EVALUATIONS * SH_FLOP_PER_TERM * sh_terms(low)
             f32 = sh_flops_per_object_step(degree) - f64
             peak = sh_flops_per_object_step(degree) / (f64 / fp64_peak + f32 / fp32_peak)
@@ -652,7 +653,7 @@ def main():
                          "unit": "TFLOP/s", "frac": achieved / peak if peak > 0 else None,
                          "traffic": per_os * steps_per_launch if per_os else None,
                          "traffic_note": "DRAM read+write bytes per launch: ncu capture of the split kernel at one "
-                                         "lane, lane-group pairs, 256-thread bound (9.8 KB per object-step: "
+                                         "lane, lane-group pairs, 256-thread bound (9.9 KB per object-step: "
                                          "local-memory write-back and epoch-record reads) times the object-steps of "
                                          "one timed launch" if per_os else None,
                          "peak_source": peak_note,
